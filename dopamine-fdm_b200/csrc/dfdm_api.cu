@@ -332,6 +332,7 @@ template <typename T> PoissonArgs<T> poisson_args(dfdm_ctx *c) {
     a.mz = metric_view<T>(c->mz_t, c->d.Nz);
     a.inv_dx = (T)(1.0 / c->dx);
     a.norm = (double)((long long)c->d.Nx * (long long)c->d.Nz);
+    a.rnorm = 1.0 / a.norm;
     a.pdiv = c->prm.dt * (3.0 / 4.0);
     a.dtp = c->dev_dt() ? c->d_dtt : nullptr;
     a.fNx = make_fastdiv((unsigned)c->d.Nx);

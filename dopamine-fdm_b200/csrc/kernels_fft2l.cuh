@@ -184,8 +184,13 @@ __device__ __forceinline__ void k_inv_x2_body(const BC &bc, const PoissonArgs<T>
 #pragma unroll
         for (int k2 = 0; k2 < N2; ++k2) {
             T2 o;
-            if (sizeof(T) == 8) { o.x = (T)((double)v[k2].x / a.norm); o.y = (T)((double)v[k2].y / a.norm); }
-            else { o.x = v[k2].x * (T)(1.0 / a.norm); o.y = v[k2].y * (T)(1.0 / a.norm); }
+            if (sizeof(T) == 8) {
+                o.x = (T)div_by((double)v[k2].x, a.norm, a.rnorm);
+                o.y = (T)div_by((double)v[k2].y, a.norm, a.rnorm);
+            } else {
+                o.x = v[k2].x * (T)a.rnorm;
+                o.y = v[k2].y * (T)a.rnorm;
+            }
             out[k1 + N1 * k2] = o;
         }
     }

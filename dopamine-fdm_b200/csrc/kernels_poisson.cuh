@@ -15,7 +15,7 @@ template <typename T> struct PoissonArgs {
     Dims d;
     Metric1D<T> my, mz;
     T inv_dx;
-    double norm;              // nxp*nzp
+    double norm, rnorm;       // nxp*nzp and its reciprocal
     double pdiv;              // dt*rk_coef(3,3)
     const double *dtp;        // adaptive time step: pdiv = dtp[0]*rk_coef(3,3) from device memory (null: fixed dt)
     FastDiv fNx, fNy, fM, fM1;   // division by Nx, Ny, Nx/2, Nx/2+1
@@ -123,16 +123,19 @@ __global__ void __launch_bounds__(256) k_col_fft(Dims d, typename cplx_t<T>::typ
             double wavenum_sum = kxx[kx] + kyy[j] + kzz[kz];
             C v = res[e];
             if (kx == 0 && j == 0 && kz == 0) { v.x = T(0); v.y = T(0); }
-            else { v.x = (T)((double)v.x / wavenum_sum); v.y = (T)((double)v.y / wavenum_sum); }
+            else {
+                const double r = 1.0 / wavenum_sum;
+                v.x = (T)div_by((double)v.x, wavenum_sum, r); v.y = (T)div_by((double)v.y, wavenum_sum, r);
+            }
             res[e] = v;
         }
         __syncthreads();
         C *other_buf = (res == b0) ? b1 : b0;
         res = fft_lines<T, true, true, TX>(res, other_buf, TX, 1, TX, p, tw);
-        const double nyp = (double)L;
+        const double nyp = (double)L, rnyp = 1.0 / nyp;
         for (int e = threadIdx.x; e < L * TX; e += blockDim.x) {
             C v = res[e];
-            v.x = (T)((double)v.x / nyp); v.y = (T)((double)v.y / nyp);
+            v.x = (T)div_by((double)v.x, nyp, rnyp); v.y = (T)div_by((double)v.y, nyp, rnyp);
             res[e] = v;
         }
         __syncthreads();
@@ -579,8 +582,8 @@ __global__ void __launch_bounds__(256) k_inv_x(PoissonArgs<T> a, int lx, const t
     for (int e = threadIdx.x; e < nl * Nx; e += blockDim.x) {
         T v = rr[e];
         T o;
-        if (sizeof(T) == 8) o = (T)((double)v / a.norm);
-        else o = v * (T)(1.0 / a.norm);
+        if (sizeof(T) == 8) o = (T)div_by((double)v, a.norm, a.rnorm);
+        else o = v * (T)a.rnorm;
         phi[line0 * Nx + e] = o;
     }
 }
@@ -615,8 +618,9 @@ __global__ void __launch_bounds__(256) k_correct(PoissonArgs<T> a, const T *__re
     }
     if (P) {
         const double pdiv = a.dtp ? *a.dtp * (3.0 / 4.0) : a.pdiv;
-        if (sizeof(T) == 8) P[p] = (T)((double)pc / pdiv);
-        else P[p] = pc * (T)(1.0 / pdiv);
+        const double rpdiv = 1.0 / pdiv;
+        if (sizeof(T) == 8) P[p] = (T)div_by((double)pc, pdiv, rpdiv);
+        else P[p] = pc * (T)rpdiv;
     }
 }
 
@@ -670,12 +674,12 @@ __device__ __forceinline__ void k_correct4_body(const BC &bc, const PoissonArgs<
     }
     if (P) {
         V4 o;
-        const double pdiv = a.dtp ? *a.dtp * (3.0 / 4.0) : a.pdiv;
+        const double pdiv = a.dtp ? *a.dtp * (3.0 / 4.0) : a.pdiv, rpdiv = 1.0 / pdiv;
         if (sizeof(T) == 8) {
-            o.x = (T)((double)pc.x / pdiv); o.y = (T)((double)pc.y / pdiv);
-            o.z = (T)((double)pc.z / pdiv); o.w = (T)((double)pc.w / pdiv);
+            o.x = (T)div_by((double)pc.x, pdiv, rpdiv); o.y = (T)div_by((double)pc.y, pdiv, rpdiv);
+            o.z = (T)div_by((double)pc.z, pdiv, rpdiv); o.w = (T)div_by((double)pc.w, pdiv, rpdiv);
         } else {
-            const T r = (T)(1.0 / pdiv);
+            const T r = (T)rpdiv;
             o.x = pc.x * r; o.y = pc.y * r; o.z = pc.z * r; o.w = pc.w * r;
         }
         *reinterpret_cast<V4 *>(P + p) = o;

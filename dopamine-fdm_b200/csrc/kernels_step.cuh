@@ -268,13 +268,13 @@ template <> struct AxisLocal<double> {
     __device__ __forceinline__ double w1m() const { return m->w1[p - 1]; }
     __device__ __forceinline__ double w0() const { return m->w0[p]; }
     __device__ __forceinline__ double w1() const { return m->w1[p]; }
-    __device__ __forceinline__ double divc(double x) const { return x / m->dc[p]; }
-    __device__ __forceinline__ double divf(double x) const { return x / m->df[p]; }
-    __device__ __forceinline__ double divfm(double x) const { return x / m->df[p - 1]; }
-    __device__ __forceinline__ double invc() const { return 1.0 / m->dc[p]; }
-    __device__ __forceinline__ double invcp() const { return 1.0 / m->dc[p + 1]; }
-    __device__ __forceinline__ double invf() const { return 1.0 / m->df[p]; }
-    __device__ __forceinline__ double invfm() const { return 1.0 / m->df[p - 1]; }
+    __device__ __forceinline__ double divc(double x) const { return div_by(x, m->dc[p], m->idc[p]); }
+    __device__ __forceinline__ double divf(double x) const { return div_by(x, m->df[p], m->idf[p]); }
+    __device__ __forceinline__ double divfm(double x) const { return div_by(x, m->df[p - 1], m->idf[p - 1]); }
+    __device__ __forceinline__ double invc() const { return m->idc[p]; }
+    __device__ __forceinline__ double invcp() const { return m->idc[p + 1]; }
+    __device__ __forceinline__ double invf() const { return m->idf[p]; }
+    __device__ __forceinline__ double invfm() const { return m->idf[p - 1]; }
 };
 
 // The gradient factor of the eddy viscosity's wall override for every wall cell (wall_gradient_factor), from the
