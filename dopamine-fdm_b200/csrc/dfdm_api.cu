@@ -374,6 +374,9 @@ int choose_kc(const Dims &d, int blocks_per_sm, int nsm, int tx = TILE_X, int ty
 }
 
 int reduce_grid(const Dims &d);
+// blocks of a column transform of `nl` columns each: the (j, kx) columns of the z transforms (families 3, 5) or the
+// (kz, kx) columns of the periodic-y solve (family 4)
+int col_blocks(const Dims &d, int which, int nl) { return (d.Nxc * (which == 4 ? d.Nz : d.Ny) + nl - 1) / nl; }
 
 template <typename T> struct Impl {
     typedef typename cplx_t<T>::type C;
@@ -941,7 +944,7 @@ template <typename T> struct Impl {
             return fwd_x(c, true, nullptr);
         case 3: case 5: {   // z transforms
             if (c->z2) {
-                dim3 g((d.Nxc + NL - 1) / NL, d.Ny);
+                const int g = col_blocks(d, which, NL);
                 with_fft2l(d.Nz, [&](auto n) {
                     constexpr int N = decltype(n)::value;
                     if (which == 3)
@@ -952,7 +955,7 @@ template <typename T> struct Impl {
                                                                               c->d_kyy, c->d_kzz);
                 });
             } else {
-                dim3 g((d.Nxc + c->tzx - 1) / c->tzx, d.Ny);
+                const int g = col_blocks(d, which, CT);
                 if (which == 3)
                     k_col_fft<T, 0, CT><<<g, 256, c->smem_z, st>>>(d, (C *)c->spec, c->plan_z, (const C *)c->tw_z, c->d_kxx, c->d_kyy, c->d_kzz);
                 else
@@ -963,14 +966,14 @@ template <typename T> struct Impl {
         }
         case 4: {   // y solve
             if (d.yper && c->y2) {
-                dim3 g((d.Nxc + NL - 1) / NL, d.Nz);
+                const int g = col_blocks(d, which, NL);
                 with_fft2l(d.Ny, [&](auto n) {
                     constexpr int N = decltype(n)::value;
                     k_col2<T, 2, NL, N><<<g, c->thr_y2, c->smem_y2, st>>>(d, (C *)c->spec, (const C *)c->tw_y, c->d_kxx,
                                                                           c->d_kyy, c->d_kzz);
                 });
             } else if (d.yper) {
-                dim3 g((d.Nxc + c->tzx - 1) / c->tzx, d.Nz);
+                const int g = col_blocks(d, which, CT);
                 k_col_fft<T, 2, CT><<<g, 256, c->smem_y, st>>>(d, (C *)c->spec, c->plan_y, (const C *)c->tw_y, c->d_kxx, c->d_kyy, c->d_kzz);
             } else if (c->ys3) {
                 const int ncol = d.Nxc * d.Nz;
@@ -3121,7 +3124,7 @@ int members_step_enqueue(const std::vector<dfdm_ctx *> &cs, cudaStream_t st,
                 if (mode == 2 && !c->yper) continue;
                 ColJob J;
                 const int L = mode == 2 ? c->d.Ny : c->d.Nz;
-                J.grid = dim3((unsigned)((c->d.Nxc + NL - 1) / NL), (unsigned)(mode == 2 ? c->d.Nz : c->d.Ny), 1);
+                J.grid = dim3((unsigned)col_blocks(c->d, mode == 2 ? 4 : 3, NL), 1, 1);
                 J.d = c->d; J.spec = (C *)c->spec; J.tw = (const C *)(mode == 2 ? c->tw_y : c->tw_z);
                 J.kxx = c->d_kxx; J.kyy = c->d_kyy; J.kzz = c->d_kzz;
                 jobs[L].push_back(J);

@@ -82,12 +82,14 @@ __global__ void __launch_bounds__(256) k_fwd_x(PoissonArgs<T> a, int lx, const T
 }
 
 // ---- 2. transforms along z (and the periodic-y Poisson solve) on column tiles ---------------------------------
-// A block loads TX consecutive kx columns of length L (rows at stride rowstride), transforms every column in
+// A block loads TX consecutive columns of length L (rows at stride rowstride), transforms every column in
 // shared memory and stores them back in place.
-//   MODE 0: forward FFT along z (rows = kz, one block per (kx tile, j))
+//   MODE 0: forward FFT along z (rows = kz, columns (j, kx))
 //   MODE 1: inverse FFT along z
-//   MODE 2: periodic y (rows = j, one block per (kx tile, kz)): forward FFT, divide by kxx+kyy+kzz with the
+//   MODE 2: periodic y (rows = j, columns (kz, kx)): forward FFT, divide by kxx+kyy+kzz with the
 //           (0,0,0) mode set to zero, inverse FFT, divide by nyp (src/projection.f90:246-273)
+// The columns are the flattened index, so only the grid's last block has columns without work: a block per (kx tile, j)
+// left Nxc mod TX columns idle in every row (Nxc = Nx/2 + 1 is never a multiple of TX).
 template <typename T, int MODE, int TX>
 __global__ void __launch_bounds__(256) k_col_fft(Dims d, typename cplx_t<T>::type *__restrict__ spec, FFTPlan p,
                                                  const typename cplx_t<T>::type *__restrict__ tw,
@@ -98,28 +100,26 @@ __global__ void __launch_bounds__(256) k_col_fft(Dims d, typename cplx_t<T>::typ
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int L = p.n;
     C *b0 = (C *)smem_raw, *b1 = b0 + L * TX;
-    const int kx0 = blockIdx.x * TX;
-    const int other = blockIdx.y;
+    // TX consecutive columns of the flattened (j, kx) index (MODE 2: (kz, kx)); a thread's elements all lie in one column
+    // (blockDim.x is a multiple of TX)
     const int Nxc = d.Nxc;
-    int base, rowstride;
-    if (MODE == 2) { base = other * d.Ny * Nxc; rowstride = Nxc; }
-    else { base = other * Nxc; rowstride = d.Ny * Nxc; }
-    for (int e = threadIdx.x; e < L * TX; e += blockDim.x) {
-        int row = e / TX, c = e % TX, kx = kx0 + c;
-        C v = mkc<T>(T(0), T(0));
-        if (kx < Nxc) v = spec[base + row * rowstride + kx];
-        b0[e] = v;
-    }
+    const int c = threadIdx.x % TX, q = blockIdx.x * TX + c;
+    const bool ok = q < Nxc * (MODE == 2 ? d.Nz : d.Ny);
+    const int rowstride = MODE == 2 ? Nxc : d.Ny * Nxc;
+    int kz = 0, kx = 0;
+    if (MODE == 2) { kz = q / Nxc; kx = q - kz * Nxc; }
+    C *col = spec + (MODE == 2 ? (size_t)kz * d.Ny * Nxc + kx : (size_t)q);
+    for (int e = threadIdx.x; e < L * TX; e += blockDim.x)
+        b0[e] = ok ? col[(size_t)(e / TX) * rowstride] : mkc<T>(T(0), T(0));
     __syncthreads();
     C *res;
     if (MODE == 0) res = fft_lines<T, false, true, TX>(b0, b1, TX, 1, TX, p, tw);
     else if (MODE == 1) res = fft_lines<T, true, true, TX>(b0, b1, TX, 1, TX, p, tw);
     else {
         res = fft_lines<T, false, true, TX>(b0, b1, TX, 1, TX, p, tw);
-        const int kz = other;
         for (int e = threadIdx.x; e < L * TX; e += blockDim.x) {
-            int j = e / TX, c = e % TX, kx = kx0 + c;
-            if (kx >= Nxc) continue;
+            const int j = e / TX;
+            if (!ok) continue;
             double wavenum_sum = kxx[kx] + kyy[j] + kzz[kz];
             C v = res[e];
             if (kx == 0 && j == 0 && kz == 0) { v.x = T(0); v.y = T(0); }
@@ -140,10 +140,8 @@ __global__ void __launch_bounds__(256) k_col_fft(Dims d, typename cplx_t<T>::typ
         }
         __syncthreads();
     }
-    for (int e = threadIdx.x; e < L * TX; e += blockDim.x) {
-        int row = e / TX, c = e % TX, kx = kx0 + c;
-        if (kx < Nxc) spec[base + row * rowstride + kx] = res[e];
-    }
+    if (ok)
+        for (int e = threadIdx.x; e < L * TX; e += blockDim.x) col[(size_t)(e / TX) * rowstride] = res[e];
 }
 
 // ---- 3. wall-bounded y: one tridiagonal system per (kx, kz) ----------------------------------------------------
