@@ -347,7 +347,8 @@ const dim3 CELL_BLOCK(32, 8, 1);
 constexpr int TILE_X = 32, TILE_Y = 8;   // (i,j) tile of the 2.5-D blocked kernels
 const int TILE_X2 = 64;   // x cells per block of the packed FP32 stage kernel (32 threads x 2 cells)
 dim3 tile_grid(const Dims &d, int kc, int tx = TILE_X) { return dim3((d.Nx + tx - 1) / tx, (d.Ny + TILE_Y - 1) / TILE_Y, (d.Nz + kc - 1) / kc); }
-// z-planes per block: enough blocks for about four waves at the measured occupancy, at most 32 planes
+// the wall kernels: one thread per wall face or cell, `sets` sets of planes
+dim3 wall_grid(const Dims &d, int sets) { return dim3((d.Nx + WALL_THREADS - 1) / WALL_THREADS, d.Nz, sets); }
 // z-planes per block of the 2.5-D tiled kernels.  A block of a (tx x ty) column runs kc planes after loading `halo`
 // extra planes; blocks_per_sm of them share an SM.  The chunking minimises (kc + halo) x g, g the waves the launch
 // takes: full waves of blocks_per_sm x nsm blocks, then a last wave as long as its most loaded SM (its blocks over
@@ -796,7 +797,7 @@ template <typename T> struct Impl {
     template <bool CORR> static int wall_factors(dfdm_ctx *c, const T *u, const T *w) {
         if (!c->d_wfac) return DFDM_OK;
         const Dims &d = c->d;
-        k_wall_sgs<T, CORR><<<dim3((d.Nx + 127) / 128, d.Nz), 128, 0, c->stream>>>(step_args<T>(c), u, w,
+        k_wall_sgs<T, CORR><<<wall_grid(d, 2), WALL_THREADS, 0, c->stream>>>(step_args<T>(c), u, w,
                                                                                    CORR ? f(c->phi) : nullptr, c->d_wfac);
         CKL();
         return DFDM_OK;
@@ -909,17 +910,14 @@ template <typename T> struct Impl {
         }
         case 8: {   // wall model (filter update at stage 1)
             if (!c->wm) return DFDM_OK;
-            dim3 g((d.Nx + 127) / 128, d.Nz);
-            int filt = c->wm_filter_mode == 1;
-            if (s == 1 && filt) {
-                k_wm_filter<T><<<g, 128, 0, st>>>(step_args<T>(c), c->wsd, f(c->u), f(c->w), c->wmf_seeded ? 0 : 1,
-                                                 c->prm.dt, c->dev_dt() ? c->d_dtt : nullptr, c->prm.wm_filter_Tf_fac);
-                CKL();
-                c->wmf_seeded = true;
-            }
+            const int filt = c->wm_filter_mode == 1;
             if (s == 1 || !filt) {   // with the filter the stress only changes with the filter (once per step)
-                k_wall_model<T><<<g, 128, 0, st>>>(step_args<T>(c), c->wsd, f(c->u), f(c->w), filt);
+                k_wall_model<T><<<wall_grid(d, 4), WALL_THREADS, 0, st>>>(step_args<T>(c), c->wsd, f(c->u), f(c->w), filt,
+                                                                          c->wmf_seeded ? 0 : 1, c->prm.dt,
+                                                                          c->dev_dt() ? c->d_dtt : nullptr,
+                                                                          c->prm.wm_filter_Tf_fac);
                 CKL();
+                if (filt) c->wmf_seeded = true;
             }
             return DFDM_OK;
         }
