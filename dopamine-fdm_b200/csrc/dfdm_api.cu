@@ -115,7 +115,7 @@ struct dfdm_ctx {
     bool fuse_ok = false, fused = false;
     void *nut = nullptr, *p = nullptr, *phi = nullptr, *spec = nullptr, *rhs3 = nullptr;
     void *my_t = nullptr, *mz_t = nullptr;      // 6 metric arrays each, storage type
-    void *zm8 = nullptr;                        // FP32: the z metrics of each plane in load8 order (StepArgs::zm8)
+    void *zm8 = nullptr;                        // FP32: the z metrics of each plane in load_pairs order (StepArgs::zm8)
     double *d_wfac = nullptr;                   // LES + wall model: wall factors of the eddy viscosity (k_wall_sgs)
     double *my_d = nullptr, *mz_d = nullptr;    // same in double
     void *tw_x = nullptr, *twr_x = nullptr, *tw_z = nullptr, *tw_y = nullptr;
@@ -292,6 +292,12 @@ template <typename T> int upload_twiddles(dfdm_ctx *c, void **dst, int n, int co
     return upload_as<T>(c, dst, h);
 }
 
+// a constant of the right-hand sides in its storage form (RhsConst)
+template <typename T> typename RhsDup<T>::type dup(double x) {
+    if constexpr (sizeof(T) == 8) return x;
+    else return make_float2((float)x, (float)x);
+}
+
 template <typename T> StepArgs<T> step_args(dfdm_ctx *c) {
     StepArgs<T> a;
     a.d = c->d;
@@ -300,13 +306,25 @@ template <typename T> StepArgs<T> step_args(dfdm_ctx *c) {
     a.myd = metric_view<double>(c->my_d, c->d.Ny);
     a.mzd = metric_view<double>(c->mz_d, c->d.Nz);
     double inv_dx = 1.0 / c->dx;
-    a.nu = (T)c->prm.nu;
     a.inv_dx = (T)inv_dx;
-    a.inv_dx2 = (T)(inv_dx * inv_dx);
     a.dx2 = (T)(c->dx * c->dx);
-    a.dPdx = (T)c->dPdx;
-    a.dPdz = (T)c->dPdz;
-    a.w_adv = (T)((c->prm.advection_scheme == 1) ? 0.0 : 0.5);
+    const double nu = c->prm.nu, wa = (c->prm.advection_scheme == 1) ? 0.0 : 0.5, wd = 1.0 - wa;
+    a.rc.inv_dx = dup<T>(inv_dx);
+    a.rc.cx = dup<T>(-0.5 * inv_dx);
+    a.rc.nu = dup<T>(nu);
+    a.rc.nu2 = dup<T>(2.0 * nu);
+    a.rc.n2x = dup<T>(2.0 * nu * (inv_dx * inv_dx));
+    a.rc.two_inv_dx2 = dup<T>(2.0 * (inv_dx * inv_dx));
+    a.rc.dPdx = dup<T>(c->dPdx);
+    a.rc.dPdz = dup<T>(c->dPdz);
+    a.rc.wd = dup<T>(wd);
+    a.rc.hwd = dup<T>(0.5 * wd);
+    a.rc.p = dup<T>(1.0 - 0.5 * wa);
+    a.rc.hp = dup<T>(0.5 - 0.25 * wa);
+    a.rc.q = dup<T>(0.5 * wa);
+    a.rc.hq = dup<T>(0.25 * wa);
+    a.rc.half = dup<T>(0.5);
+    a.rc.m2 = dup<T>(-2.0);
     a.nwl = c->nwl;
     a.wm = c->wm;
     a.sgs_model = c->prm.sgs_model;
@@ -624,15 +642,10 @@ template <typename T> struct Impl {
         int dev = 0, nsm = 148, occ = 1;
         CK(cudaGetDevice(&dev));
         CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        const void *stage_fn;
-        if constexpr (sizeof(T) == 8)
-            stage_fn = c->les ? (const void *)k_tiled<T, true, true, TILE_X, TILE_Y, 0>
-                              : (const void *)k_tiled<T, false, true, TILE_X, TILE_Y, 0>;
-        else
-            stage_fn = c->les ? (c->wm ? (const void *)k_tiled<T, true, true, TILE_X, TILE_Y, 0>
-                                       : (const void *)k_tiled<T, true, false, TILE_X, TILE_Y, 0>)
-                              : (c->wm ? (const void *)k_tiled<T, false, true, TILE_X, TILE_Y, 0>
-                                       : (const void *)k_tiled<T, false, false, TILE_X, TILE_Y, 0>);
+        const void *stage_fn = c->les ? (c->wm ? (const void *)k_tiled<T, true, true, TILE_X, TILE_Y, 0>
+                                               : (const void *)k_tiled<T, true, false, TILE_X, TILE_Y, 0>)
+                                      : (c->wm ? (const void *)k_tiled<T, false, true, TILE_X, TILE_Y, 0>
+                                               : (const void *)k_tiled<T, false, false, TILE_X, TILE_Y, 0>);
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, stage_fn, TILE_X * TILE_Y, 0));
         c->kc_stage = choose_kc(d, occ, nsm);
         if constexpr (sizeof(T) == 4) {
@@ -818,21 +831,12 @@ template <typename T> struct Impl {
         else return c->wm ? les_launch<true, CORR>(c, sc) : les_launch<false, CORR>(c, sc);
     }
     template <bool HYB> static int stage_dispatch(dfdm_ctx *c, const StageCoef &sc, T *rhs_only) {
-        if constexpr (sizeof(T) == 8) {   // FP64 keeps the runtime wall-model flag
-            return c->les ? stage_launch<true, true, HYB, false>(c, sc, rhs_only) : stage_launch<false, true, HYB, false>(c, sc, rhs_only);
-        } else {
-            if (c->les) {
-                if (c->wm) return stage_launch<true, true, HYB, false>(c, sc, rhs_only); else return stage_launch<true, false, HYB, false>(c, sc, rhs_only);
-            } else {
-                if (c->wm) return stage_launch<false, true, HYB, false>(c, sc, rhs_only); else return stage_launch<false, false, HYB, false>(c, sc, rhs_only);
-            }
-        }
+        if (c->les) return c->wm ? stage_launch<true, true, HYB, false>(c, sc, rhs_only) : stage_launch<true, false, HYB, false>(c, sc, rhs_only);
+        return c->wm ? stage_launch<false, true, HYB, false>(c, sc, rhs_only) : stage_launch<false, false, HYB, false>(c, sc, rhs_only);
     }
     // stages 2 and 3 with the fused correction (no hybrid scheme: fuse_eligible; LES goes through les_dispatch)
     static int stage_dispatch_corr(dfdm_ctx *c, const StageCoef &sc) {
-        if constexpr (sizeof(T) == 8) return stage_launch<false, true, false, true>(c, sc, nullptr);
-        else if (c->wm) return stage_launch<false, true, false, true>(c, sc, nullptr);
-        else return stage_launch<false, false, false, true>(c, sc, nullptr);
+        return c->wm ? stage_launch<false, true, false, true>(c, sc, nullptr) : stage_launch<false, false, false, true>(c, sc, nullptr);
     }
 
     static int stage_kernel(dfdm_ctx *c, const StageCoef &sc, T *rhs_only) {
@@ -1631,12 +1635,13 @@ int dfdm_create(const dfdm_grid *g, const dfdm_params *prm, dfdm_ctx **out) {
         if ((rc = upload_as<float>(c, &c->my_t, my))) return bail(rc);
         if ((rc = upload_as<float>(c, &c->mz_t, mz))) return bail(rc);
         // per plane k: w0(k-1), w1(k-1), w0(k), w1(k), idc(k), idc(k+1), idf(k-1), idf(k) of metric_view's layout
-        // (AxisLocal<F2>::metric_src), the same FP32 values as mz_t
+        // (AxisLocal<F2>::load_pairs), each twice, the same FP32 values as mz_t
         const int L = d.Nz + 3;
-        std::vector<double> z8((size_t)d.Nz * 8);
+        std::vector<double> z8((size_t)d.Nz * ZPAIRS);
         for (int k = 0; k < d.Nz; ++k) {
             const int src[8][2] = {{2, k - 1}, {3, k - 1}, {2, k}, {3, k}, {4, k}, {4, k + 1}, {5, k - 1}, {5, k}};
-            for (int t = 0; t < 8; ++t) z8[(size_t)k * 8 + t] = mz[(size_t)src[t][0] * L + 1 + src[t][1]];
+            for (int t = 0; t < 8; ++t)
+                z8[(size_t)k * ZPAIRS + 2 * t] = z8[(size_t)k * ZPAIRS + 2 * t + 1] = mz[(size_t)src[t][0] * L + 1 + src[t][1]];
         }
         if ((rc = upload_as<float>(c, &c->zm8, z8))) return bail(rc);
     }

@@ -6,14 +6,55 @@
 
 namespace dfdm {
 
+// Elementwise arithmetic of the right-hand sides for double, float and packed pairs: one fused multiply-add where the
+// formulas below say mad / nmad.
+__device__ __forceinline__ double mad(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float mad(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ F2 mad(F2 a, F2 b, F2 c) { return F2(__ffma2_rn(a.v, b.v, c.v)); }
+template <typename T> __device__ __forceinline__ T nmad(T a, T b, T c) { return mad(-a, b, c); }   // c - a b
+__device__ __forceinline__ double mulv(double a, double b) { return a * b; }
+__device__ __forceinline__ float mulv(float a, float b) { return a * b; }
+__device__ __forceinline__ F2 mulv(F2 a, F2 b) { return F2(__fmul2_rn(a.v, b.v)); }
+
+// The constants of the right-hand sides.  FP32 keeps each twice, so that a packed kernel reads a pair with one load.
+template <typename D> struct RhsConst {
+    D inv_dx, cx, nu, nu2, n2x, two_inv_dx2, dPdx, dPdz;   // 1/dx, -1/(2 dx), nu, 2 nu, 2 nu/dx^2, 2/dx^2
+    D wd, p, q, hwd, hp, hq;                   // the blend outside the wall band: wd = 1 - wa, p = 1 - wa/2, q = wa/2, halves
+    D half, m2;                                // 0.5, -2
+};
+template <typename T> struct RhsDup;
+template <> struct RhsDup<double> { typedef double type; };
+template <> struct RhsDup<float> { typedef float2 type; };
+template <typename T> __device__ __forceinline__ T bcast(double x) { return T(x); }
+template <typename T> __device__ __forceinline__ T bcast(float2 x);
+template <> __device__ __forceinline__ float bcast<float>(float2 x) { return x.x; }
+template <> __device__ __forceinline__ F2 bcast<F2>(float2 x) { return F2(x); }
+
+// Base-profile terms of one row (FP32; the profile is zero in FP64), from ub of rows j-1, j, j+1 (mirrored on wall ghost
+// rows).  f, fm: the profile at the y faces j and j-1; x: (1 + wd) ub; c: its diffusion's flux difference; dp, dm: its steps
+// across the two faces.
+template <typename T> struct RowProfile {
+    T u, f, fm, x, c, dp, dm;
+    template <typename Y> __device__ __forceinline__ void load(const T *ubr, const Y &y, T wd) {
+        u = ubr[1];
+        f = mad(y.w1(), ubr[2], mulv(y.w0(), ubr[1]));
+        fm = mad(y.w1m(), ubr[1], mulv(y.w0m(), ubr[0]));
+        x = mad(wd, ubr[1], ubr[1]);
+        dp = ubr[2] - ubr[1];
+        dm = ubr[1] - ubr[0];
+        c = nmad(y.invfm(), dm, mulv(y.invf(), dp));
+    }
+};
+template <> struct RowProfile<double> {
+    template <typename Y> __device__ __forceinline__ void load(const double *, const Y &, double) {}
+};
+
 // Everything a step kernel reads besides the fields.  Metric arrays are offset so index -1 is valid.
 template <typename T> struct StepArgs {
     Dims d;
     Metric1D<T> my, mz;          // y and z metrics in the storage type
     Metric1D<double> myd, mzd;   // the same in double (wall model, reductions)
-    T nu, inv_dx, inv_dx2, dx2;
-    T dPdx, dPdz;
-    T w_adv;                     // 0.5 skew-symmetric, 0 divergence form
+    T inv_dx, dx2;
     int nwl;                     // divergence-form wall band (adv_wall_layers)
     int wm;                      // flat-wall EQWM on both no-slip walls
     int sgs_model;               // 1 Vreman, 2 AMD
@@ -29,8 +70,9 @@ template <typename T> struct StepArgs {
     // fused correction of the previous stage (CORR kernels): its potential phi; the plane loads then hold u* and
     // the loader forms u = u* - grad(phi) exactly as k_correct does
     const T *phi;
-    // FP32: the eight z metrics of every plane in AxisLocal<F2>::load8 order, 8 consecutive values per plane (one
-    // 32-byte bulk copy per plane for the TMA stage kernel); null in FP64
+    RhsConst<typename RhsDup<T>::type> rc;
+    // FP32: the eight z metrics of every plane in AxisLocal<F2>::load_pairs order, each twice: ZPAIRS consecutive values
+    // per plane (copied to shared memory with the plane); null in FP64
     const float *zm8;
     // LES with the wall model: the first-cell gradient factor of every wall cell, (iw*Nz + k)*Nx + i, written by
     // k_wall_sgs from the velocity the eddy viscosity is computed from (NaN where the override does not apply);
@@ -185,7 +227,8 @@ __global__ void __launch_bounds__(WALL_THREADS) k_wall_model(StepArgs<T> a, Wall
 // ---------------------------------------------------------------------------------------------------------------
 // Metric values around one index p of an axis: weights of faces p-1 and p, widths and spacings at p-1, p, p+1.
 // FP32 reads them once per thread (y) or once per plane (z) and keeps them in registers; FP64 reads them where
-// they are used (its registers are taken by the double-precision stencil) and divides exactly, as Arith does.
+// they are used (its registers are taken by the double-precision stencil).
+constexpr int ZPAIRS = 16;   // floats of one plane's z metrics in load_pairs order
 template <typename T> struct AxisLocal;
 template <> struct AxisLocal<float> {
     float w0m_, w1m_, w0_, w1_, idc_, idcp_, idfm_, idf_;
@@ -197,9 +240,6 @@ template <> struct AxisLocal<float> {
     __device__ __forceinline__ float w1m() const { return w1m_; }
     __device__ __forceinline__ float w0() const { return w0_; }
     __device__ __forceinline__ float w1() const { return w1_; }
-    __device__ __forceinline__ float divc(float x) const { return x * idc_; }
-    __device__ __forceinline__ float divf(float x) const { return x * idf_; }
-    __device__ __forceinline__ float divfm(float x) const { return x * idfm_; }
     __device__ __forceinline__ float invc() const { return idc_; }
     __device__ __forceinline__ float invcp() const { return idcp_; }
     __device__ __forceinline__ float invf() const { return idf_; }
@@ -211,31 +251,17 @@ template <> struct AxisLocal<F2> {   // packed pairs: the same metrics broadcast
         w0m_ = F2(__ldg(m.w0 + p - 1)); w1m_ = F2(__ldg(m.w1 + p - 1)); w0_ = F2(__ldg(m.w0 + p)); w1_ = F2(__ldg(m.w1 + p));
         idc_ = F2(__ldg(m.idc + p)); idcp_ = F2(__ldg(m.idc + p + 1)); idfm_ = F2(__ldg(m.idf + p - 1)); idf_ = F2(__ldg(m.idf + p));
     }
-    // the same eight values staged by metric_src (w0, w1 at p-1 and p; idc at p, p+1; idf at p-1, p)
-    __device__ __forceinline__ void load8(const float *z) {
-        w0m_ = F2(z[0]); w1m_ = F2(z[1]); w0_ = F2(z[2]); w1_ = F2(z[3]);
-        idc_ = F2(z[4]); idcp_ = F2(z[5]); idfm_ = F2(z[6]); idf_ = F2(z[7]);
-    }
-    // the address of staged value t (0..7) of point p, in the order of load8
-    static __device__ __forceinline__ const float *metric_src(const Metric1D<float> &m, int p, int t) {
-        switch (t) {
-        case 0: return m.w0 + p - 1;
-        case 1: return m.w1 + p - 1;
-        case 2: return m.w0 + p;
-        case 3: return m.w1 + p;
-        case 4: return m.idc + p;
-        case 5: return m.idc + p + 1;
-        case 6: return m.idf + p - 1;
-        default: return m.idf + p;
-        }
+    // the same eight values, each twice (w0, w1 at p-1 and p; idc at p, p+1; idf at p-1, p), from 16-byte aligned storage
+    __device__ __forceinline__ void load_pairs(const float *z) {
+        const float4 *z4 = reinterpret_cast<const float4 *>(z);
+        const float4 a = z4[0], b = z4[1], c = z4[2], e = z4[3];
+        w0m_ = F2::pair(a.x, a.y); w1m_ = F2::pair(a.z, a.w); w0_ = F2::pair(b.x, b.y); w1_ = F2::pair(b.z, b.w);
+        idc_ = F2::pair(c.x, c.y); idcp_ = F2::pair(c.z, c.w); idfm_ = F2::pair(e.x, e.y); idf_ = F2::pair(e.z, e.w);
     }
     __device__ __forceinline__ F2 w0m() const { return w0m_; }
     __device__ __forceinline__ F2 w1m() const { return w1m_; }
     __device__ __forceinline__ F2 w0() const { return w0_; }
     __device__ __forceinline__ F2 w1() const { return w1_; }
-    __device__ __forceinline__ P2 divc(F2 x) const { return x * idc_; }
-    __device__ __forceinline__ P2 divf(F2 x) const { return x * idf_; }
-    __device__ __forceinline__ P2 divfm(F2 x) const { return x * idfm_; }
     __device__ __forceinline__ F2 invc() const { return idc_; }
     __device__ __forceinline__ F2 invcp() const { return idcp_; }
     __device__ __forceinline__ F2 invf() const { return idf_; }
@@ -249,9 +275,6 @@ template <> struct AxisLocal<double> {
     __device__ __forceinline__ double w1m() const { return m->w1[p - 1]; }
     __device__ __forceinline__ double w0() const { return m->w0[p]; }
     __device__ __forceinline__ double w1() const { return m->w1[p]; }
-    __device__ __forceinline__ double divc(double x) const { return div_by(x, m->dc[p], m->idc[p]); }
-    __device__ __forceinline__ double divf(double x) const { return div_by(x, m->df[p], m->idf[p]); }
-    __device__ __forceinline__ double divfm(double x) const { return div_by(x, m->df[p - 1], m->idf[p - 1]); }
     __device__ __forceinline__ double invc() const { return m->idc[p]; }
     __device__ __forceinline__ double invcp() const { return m->idc[p + 1]; }
     __device__ __forceinline__ double invf() const { return m->idf[p]; }
@@ -292,198 +315,212 @@ __global__ void __launch_bounds__(WALL_THREADS) k_wall_sgs(StepArgs<T> a, const 
 template <typename T> __device__ __forceinline__ T wall_flux(const double *t) { return (T)t[0]; }
 template <> __device__ __forceinline__ F2 wall_flux<F2>(const double *t) { return F2::pair((float)t[0], (float)t[1]); }
 
-// Right-hand sides (src/equations.f90), evaluated in the reference's expression order at one index (i,j,k).
-// `q` is a neighbourhood accessor: q.U(di,dj,dk) is U at (i+di, j+dj, k+dk) with every boundary rule already
-// applied (periodic wraps, no-slip mirror, zero wall faces, zero nu_t ghosts), so the formulas below see the
-// same values the reference reads from its ghosted arrays.
-template <typename T, bool LES, bool WM, typename Q, typename SA>
-__device__ __forceinline__ T rhs_u_at(const SA &a, const Q &q, const AxisLocal<T> &Y, const AxisLocal<T> &Z,
-                                    const double *__restrict__ tau_x, int i, int j, int k) {
+// The right-hand sides of u, v and w (src/equations.f90:25-721) at one index (i, j, k), from the neighbourhood accessor q
+// (q.Ud: U as stored, the deviation from the row's base profile; equal to U in FP64).  Every boundary rule is applied in q
+// and the profile terms, so the formulas see the values the reference reads from its ghosted arrays.
+//
+// The reference writes each convective term as wd (a1 b1 - a0 b0) + wa b (a1 - a0), a the advected and b the advecting
+// velocity on the two faces, b = (b0 + b1)/2 and wa + wd = 1 (wa = 1/2 skew-symmetric, 0 divergence form and in the wall
+// band).  It is evaluated here in the equivalent forms with the fewest operations:
+//   a1 (wd b1 + m) - a0 (wd b0 + m), m = wa (b0 + b1)/2              where a1 - a0 needs no care,
+//   (wd b1 or a's total) (b1 - b0) + (a1 - a0)(p b0 + q b1)           where U is the one interpolated: FP32 then takes
+//     a1 - a0 from the stored deviations, without the cancellation of the mean flow,
+//   (a1 - a0) (wd (a1 + a0) + wa a)                                  for uu, vv, ww,
+// interpolations to the y face j and the z face k are shared by two equations each, with constant viscosity the two terms of
+// a flux are collected before its metric, and with an eddy viscosity each edge's shear flux is formed once.  About 160
+// operations per cell against 240 for the term by term form (which in FP64 had 24 divisions besides), and in FP64 with a
+// smaller error against 80-bit arithmetic (relative to a noisy channel's right-hand sides: u 1.8e-15 -> 1.4e-16, v and w
+// 1.7e-16 -> 1.6e-16), since fewer terms are rounded.  The stage kernels are bound by instruction issue at 16 warps per SM:
+// 256 x 192 x 256 cells went from 172 to 146 us (stage 1) and from 223 to 187 us (fused stage) in FP32, and the FP64 step
+// from 2.74 to 2.41 ms; the LES kernels on 96 x 64 x 96 cells take 20 us as before in FP32, 90 x 53 x 60 cells step in 195
+// against 224 us in FP64.
+template <typename T, bool LES, bool WM, typename Q, typename SA, typename ZM>
+__device__ __forceinline__ void rhs_at(const SA &a, const Q &q, const AxisLocal<T> &Y, const RowProfile<T> &R, const ZM &Z,
+                                       const double *__restrict__ tau_x, const double *__restrict__ tau_z, int i, int j,
+                                       int k, bool vrow, T &ru, T &rv, T &rw) {
+    constexpr bool PROF = Fp32Forms<T>::value;
     const Dims &d = a.d;
-    T Uc = q.U(0, 0, 0), Uim = q.U(-1, 0, 0), Uip = q.U(1, 0, 0);
-    T Ujm = q.U(0, -1, 0), Ujp = q.U(0, 1, 0), Ukm = q.U(0, 0, -1), Ukp = q.U(0, 0, 1);
-    bool wm_band = WM && a.wm && (j + 2 <= 1 + a.nwl || j + 2 >= d.Ny + 2 - a.nwl);
-    T wa = wm_band ? T(0) : a.w_adv, wd = T(1) - wa;
-    // -d(uu)/dx
-    T r;
-    if constexpr (Fp32Forms<T>::value) {
-        // FP32: t1^2 - t0^2 = (t1 - t0)(t1 + t0) with t1 - t0 from the stored deviations (no cancellation)
-        T dlt = T(0.5) * (q.Ud(1, 0, 0) - q.Ud(-1, 0, 0));
-        T sum = T(0.5) * (Uip + Uim) + Uc;
-        r = -dlt * (wd * sum + wa * Uc) * a.inv_dx;
-    } else {
-        T t1 = T(0.5) * (Uc + Uip), t0 = T(0.5) * (Uim + Uc);
-        r = -(wd * (t1 * t1 - t0 * t0) + wa * Uc * (t1 - t0)) * a.inv_dx;
+    const auto &K = a.rc;
+    const T inv_dx = bcast<T>(K.inv_dx), half = bcast<T>(K.half), m2 = bcast<T>(K.m2), nu = bcast<T>(K.nu);
+    const T wd0 = bcast<T>(K.wd), q0 = bcast<T>(K.q), hwd0 = bcast<T>(K.hwd), p0 = bcast<T>(K.p);   // v: never banded
+    T wd = wd0, hwd = hwd0, pp = p0, qq = q0, hp = bcast<T>(K.hp), hq = bcast<T>(K.hq);
+    if (WM && a.wm && (j < a.nwl || j >= d.Ny - a.nwl)) {   // divergence form in the wall band
+        wd = T(1); hwd = T(0.5); pp = T(1); qq = T(0); hp = T(0.5); hq = T(0);
     }
-    // -d(uv)/dy: u at y faces j-1, j (weighted), v at x faces (plain average)
-    T V00 = q.V(0, 0, 0), V10 = q.V(1, 0, 0), V0m = q.V(0, -1, 0), V1m = q.V(1, -1, 0);
+    const bool wall_lo = WM && a.wm && j == 0, wall_hi = WM && a.wm && j == d.Ny - 1;
+    const bool in_lo = d.yper != 0 || j != 0, in_hi = d.yper != 0 || j != d.Ny - 1;   // LES: nu_t reaches the face
+    (void)wall_lo; (void)wall_hi; (void)in_lo; (void)in_hi;
+    auto N = [&](int di, int dj, int dk) { return q.N(di, dj, dk); };
+
+    // Values that two equations share are written out in both: the compiler keeps them in registers, except in the LES
+    // kernels, where SEP makes it read the shared planes again instead (their registers are full: it would spill).
+    auto SEP = [] { if constexpr (LES) asm volatile("" ::: "memory"); };
+    // LES: the shear fluxes through the upper edges, (nu + nu_t)(dU_a/dx_b + dU_b/dx_a), serve two equations each
+    T fxy = T(0), fxz = T(0), fyz = T(0);
+    (void)fxy; (void)fxz; (void)fyz;
+    // ---- u ----
     {
-        T u1 = Y.w0() * Uc + Y.w1() * Ujp, u0 = Y.w0m() * Ujm + Y.w1m() * Uc;
-        T v1 = T(0.5) * (V00 + V10), v0 = T(0.5) * (V0m + V1m);
-        r = r - Y.divc(wd * (u1 * v1 - u0 * v0) + wa * T(0.5) * (v0 + v1) * (u1 - u0));
-    }
-    // -d(uw)/dz
-    T W00 = q.W(0, 0, 0), W10 = q.W(1, 0, 0), W0m = q.W(0, 0, -1), W1m = q.W(1, 0, -1);
-    {
-        T u1 = Z.w0() * Uc + Z.w1() * Ukp, u0 = Z.w0m() * Ukm + Z.w1m() * Uc;
-        T w1 = T(0.5) * (W00 + W10), w0 = T(0.5) * (W0m + W1m);
-        if constexpr (Fp32Forms<T>::value) {
-            // u1 w1 - u0 w0 = u1 (w1 - w0) + w0 (u1 - u0); u1 - u0 from deviations (same row: the profile cancels)
-            T Udc = q.Ud(0, 0, 0);
-            T du = (Z.w0() * Udc + Z.w1() * q.Ud(0, 0, 1)) - (Z.w0m() * q.Ud(0, 0, -1) + Z.w1m() * Udc);
-            r = r - Z.divc(wd * (u1 * (w1 - w0) + w0 * du) + wa * T(0.5) * (w0 + w1) * du);
+        const T Uc = q.Ud(0, 0, 0), Vc = q.V(0, 0, 0), Wc = q.W(0, 0, 0), Ujp = q.Ud(0, 1, 0), Ukp = q.Ud(0, 0, 1);
+        const T V10 = q.V(1, 0, 0), W10 = q.W(1, 0, 0);
+        const T uy = mad(Y.w1(), Ujp, mulv(Y.w0(), Uc)), uz = mad(Z.w1(), Ukp, mulv(Z.w0(), Uc));   // to y face j, z face k
+        const T dUy = Ujp - Uc, dUz = Ukp - Uc, dVx = V10 - Vc, dWx = W10 - Wc;
+        const T Um = q.Ud(-1, 0, 0), Up = q.Ud(1, 0, 0), s = Up + Um;
+        T e;
+        if constexpr (PROF) e = mad(hwd, s, Uc + R.x); else e = mad(hwd, s, Uc);
+        T r = mad(mulv(bcast<T>(K.cx), Up - Um), e, bcast<T>(K.dPdx));
+        const T V0m = q.V(0, -1, 0), V1m = q.V(1, -1, 0), Ujm = q.Ud(0, -1, 0);
+        const T W0m = q.W(0, 0, -1), W1m = q.W(1, 0, -1), Ukm = q.Ud(0, 0, -1);
+        // y
+        const T vs1 = Vc + V10, vs0 = V0m + V1m, m = mulv(hq, vs0 + vs1);
+        T u1, u0;
+        if constexpr (PROF) { u1 = uy + R.f; u0 = mad(Y.w1m(), Uc, mad(Y.w0m(), Ujm, R.fm)); }
+        else { u1 = uy; u0 = mad(Y.w1m(), Uc, mulv(Y.w0m(), Ujm)); }
+        const T cy = nmad(u0, mad(hwd, vs0, m), mulv(u1, mad(hwd, vs1, m)));
+        // z
+        const T ws1 = Wc + W10, ws0 = W0m + W1m, uzm = mad(Z.w1m(), Uc, mulv(Z.w0m(), Ukm)), du = uz - uzm;
+        T ut;
+        if constexpr (PROF) ut = uz + R.u; else ut = uz;
+        const T cz = mad(du, mad(hq, ws1, mulv(hp, ws0)), mulv(mulv(hwd, ut), ws1 - ws0));
+        if constexpr (LES || WM) {
+            T nx1 = nu, nx2 = nu, ny1 = nu, ny2 = nu, nz1 = nu, nz2 = nu;
+            if constexpr (LES) {
+                const T n0 = N(0, 0, 0), n1 = N(1, 0, 0), ns = n0 + n1;
+                nx1 = nu + n0; nx2 = nu + n1;
+                if (in_lo) ny1 = mad(half, mad(Y.w0m(), N(0, -1, 0) + N(1, -1, 0), mulv(Y.w1m(), ns)), nu);
+                if (in_hi) ny2 = mad(half, mad(Y.w1(), N(0, 1, 0) + N(1, 1, 0), mulv(Y.w0(), ns)), nu);
+                nz1 = mad(half, mad(Z.w0m(), N(0, 0, -1) + N(1, 0, -1), mulv(Z.w1m(), ns)), nu);
+                nz2 = mad(half, mad(Z.w1(), N(0, 0, 1) + N(1, 0, 1), mulv(Z.w0(), ns)), nu);
+            }
+            T sp = dUy, sm = Uc - Ujm;
+            if constexpr (PROF) { sp = sp + R.dp; sm = sm + R.dm; }
+            T fy2 = mulv(ny2, mad(Y.invf(), sp, mulv(inv_dx, dVx)));
+            T fy1 = mulv(ny1, mad(Y.invfm(), sm, mulv(inv_dx, V1m - V0m)));
+            const T fz2 = mulv(nz2, mad(Z.invf(), dUz, mulv(inv_dx, dWx)));
+            fxy = fy2; fxz = fz2;
+            if (wall_lo) fy1 = wall_flux<T>(tau_x + k * d.Nx + i);
+            if (wall_hi) fy2 = wall_flux<T>(tau_x + (d.Nz + k) * d.Nx + i);
+            const T fz1 = mulv(nz1, mad(Z.invfm(), Uc - Ukm, mulv(inv_dx, W1m - W0m)));
+            const T fx = nmad(nx1, Uc - Um, mulv(nx2, Up - Uc));
+            r = mad(bcast<T>(K.two_inv_dx2), fx, r);
+            r = mad(Y.invc(), (fy2 - fy1) - cy, r);
+            ru = mad(Z.invc(), (fz2 - fz1) - cz, r);
         } else {
-            r = r - Z.divc(wd * (u1 * w1 - u0 * w0) + wa * T(0.5) * (w0 + w1) * (u1 - u0));
+            r = mad(bcast<T>(K.n2x), mad(m2, Uc, s), r);
+            T F;
+            if constexpr (PROF) F = mad(Y.invf(), dUy, R.c); else F = mulv(Y.invf(), dUy);
+            F = mad(inv_dx, dVx - (V1m - V0m), nmad(Y.invfm(), Uc - Ujm, F));
+            r = mad(Y.invc(), mad(nu, F, -cy), r);
+            F = nmad(Z.invfm(), Uc - Ukm, mulv(Z.invf(), dUz));
+            F = mad(inv_dx, dWx - (W1m - W0m), F);
+            ru = mad(Z.invc(), mad(nu, F, -cz), r);
         }
     }
-    // viscous: d(2 nu_x du/dx)/dx + d(nu_y (du/dy + dv/dx))/dy + d(nu_z (du/dz + dw/dx))/dz + dPdx
-    T inv_dz3 = Z.invc(), inv_dy3 = Y.invc();
-    T nu = a.nu;
-    T nu_x1 = nu, nu_x2 = nu, nu_y1 = nu, nu_y2 = nu, nu_z1 = nu, nu_z2 = nu;
-    if (LES) {
-        T n_c = q.N(0, 0, 0), n_p = q.N(1, 0, 0);
-        nu_x1 = nu + n_c; nu_x2 = nu + n_p;
-        if (!(d.yper == 0 && j == 0))
-            nu_y1 = nu + T(0.5) * (Y.w0m() * q.N(0, -1, 0) + Y.w1m() * n_c + Y.w0m() * q.N(1, -1, 0) + Y.w1m() * n_p);
-        if (!(d.yper == 0 && j == d.Ny - 1))
-            nu_y2 = nu + T(0.5) * (Y.w0() * n_c + Y.w1() * q.N(0, 1, 0) + Y.w0() * n_p + Y.w1() * q.N(1, 1, 0));
-        nu_z1 = nu + T(0.5) * (Z.w0m() * (q.N(0, 0, -1) + q.N(1, 0, -1)) + Z.w1m() * (n_c + n_p));
-        nu_z2 = nu + T(0.5) * (Z.w0() * (n_c + n_p) + Z.w1() * (q.N(0, 0, 1) + q.N(1, 0, 1)));
+    // ---- v ----
+    rv = T(0);
+    if (vrow) {
+        SEP();
+        const T Uc = q.Ud(0, 0, 0), Vc = q.V(0, 0, 0), Wc = q.W(0, 0, 0), Ujp = q.Ud(0, 1, 0), Wjp = q.W(0, 1, 0);
+        const T V10 = q.V(1, 0, 0), Vkp = q.V(0, 0, 1);
+        const T uy = mad(Y.w1(), Ujp, mulv(Y.w0(), Uc)), wy = mad(Y.w1(), Wjp, mulv(Y.w0(), Wc));   // to y face j
+        const T vz = mad(Z.w1(), Vkp, mulv(Z.w0(), Vc));                                             // to z face k
+        const T dUy = Ujp - Uc, dWy = Wjp - Wc, dVx = V10 - Vc, dVz = Vkp - Vc;
+        const T Vjp = q.V(0, 1, 0), Vjm = q.V(0, -1, 0), Vm = q.V(-1, 0, 0), Vkm = q.V(0, 0, -1);
+        const T Um = q.Ud(-1, 0, 0), Ump = q.Ud(-1, 1, 0), Wkm = q.W(0, 0, -1), Wkmjp = q.W(0, 1, -1);
+        // y
+        const T ey = mulv(mulv(half, Vjp - Vjm), mad(hwd0, Vjp + Vjm, Vc));
+        // x
+        const T um = mad(Y.w1(), Ump, mulv(Y.w0(), Um)), du = uy - um, vs = Vm + Vc;
+        T g;
+        if constexpr (PROF) g = mad(q0, um, mad(p0, uy, R.f)); else g = mad(q0, um, mulv(p0, uy));
+        const T cx = mad(mulv(hwd0, vs), du, mulv(mulv(half, V10 - Vm), g));
+        // z
+        const T vzm = mad(Z.w1m(), Vc, mulv(Z.w0m(), Vkm)), wym = mad(Y.w1(), Wkmjp, mulv(Y.w0(), Wkm));
+        const T m = mulv(q0, wym + wy);
+        const T cz = nmad(vzm, mad(wd0, wym, m), mulv(vz, mad(wd0, wy, m)));
+        if constexpr (LES) {
+            const T n0 = N(0, 0, 0), np = N(0, 1, 0), w0 = Y.w0(), w1 = Y.w1(), ny = mad(w1, np, mulv(w0, n0));
+            const T nx1 = mad(half, mad(w1, N(-1, 1, 0), mad(w0, N(-1, 0, 0), ny)), nu);
+            const T nz1 = mad(Z.w0m(), mad(w1, N(0, 1, -1), mulv(w0, N(0, 0, -1))), mad(Z.w1m(), ny, nu));
+            const T nz2 = mad(Z.w1(), mad(w1, N(0, 1, 1), mulv(w0, N(0, 0, 1))), mad(Z.w0(), ny, nu));
+            T un = Ump - Um;   // the total across the y face (with constant viscosity the profile's step cancels)
+            if constexpr (PROF) un = un + R.dp;
+            const T fx1 = mulv(nx1, mad(inv_dx, Vc - Vm, mulv(Y.invf(), un)));
+            const T fz2 = mulv(nz2, mad(Z.invf(), dVz, mulv(Y.invf(), dWy)));
+            fyz = fz2;
+            const T fz1 = mulv(nz1, mad(Z.invfm(), Vc - Vkm, mulv(Y.invf(), Wkmjp - Wkm)));
+            const T fy = nmad(nu + n0, mulv(Y.invc(), Vc - Vjm), mulv(nu + np, mulv(Y.invcp(), Vjp - Vc)));
+            T r = mulv(Y.invf(), mad(fy, T(2), -ey));
+            r = mad(inv_dx, (fxy - fx1) - cx, r);
+            rv = mad(Z.invc(), (fz2 - fz1) - cz, r);
+        } else {
+            T F = nmad(Y.invc(), Vc - Vjm, mulv(Y.invcp(), Vjp - Vc));
+            T r = mulv(Y.invf(), mad(bcast<T>(K.nu2), F, -ey));
+            F = mad(Y.invf(), dUy - (Ump - Um), mulv(inv_dx, mad(m2, Vc, V10 + Vm)));
+            r = mad(inv_dx, mad(nu, F, -cx), r);
+            F = nmad(Z.invfm(), Vc - Vkm, mulv(Z.invf(), dVz));
+            F = mad(Y.invf(), dWy - (Wkmjp - Wkm), F);
+            rv = mad(Z.invc(), mad(nu, F, -cz), r);
+        }
     }
-    T tj = Y.divf(Ujp - Uc), tjm = Y.divfm(Uc - Ujm);
-    T fy2 = nu_y2 * (tj + (V10 - V00) * a.inv_dx);
-    T fy1 = nu_y1 * (tjm + (V1m - V0m) * a.inv_dx);
-    if (WM && a.wm) {
-        if (j == 0) fy1 = wall_flux<T>(tau_x + k * d.Nx + i);
-        if (j == d.Ny - 1) fy2 = wall_flux<T>(tau_x + (d.Nz + k) * d.Nx + i);
+    // ---- w ----
+    {
+        SEP();
+        const T Uc = q.Ud(0, 0, 0), Vc = q.V(0, 0, 0), Wc = q.W(0, 0, 0), Ukp = q.Ud(0, 0, 1), Wjp = q.W(0, 1, 0);
+        const T W10 = q.W(1, 0, 0), Vkp = q.V(0, 0, 1);
+        const T uz = mad(Z.w1(), Ukp, mulv(Z.w0(), Uc)), vz = mad(Z.w1(), Vkp, mulv(Z.w0(), Vc));   // to z face k
+        const T wy = mad(Y.w1(), Wjp, mulv(Y.w0(), Wc));                                             // to y face j
+        const T dUz = Ukp - Uc, dVz = Vkp - Vc, dWy = Wjp - Wc, dWx = W10 - Wc;
+        const T Wkp = q.W(0, 0, 1), Wkm = q.W(0, 0, -1), Wm = q.W(-1, 0, 0), Wjm = q.W(0, -1, 0);
+        const T Um = q.Ud(-1, 0, 0), Umkp = q.Ud(-1, 0, 1), Vjm = q.V(0, -1, 0), Vjmkp = q.V(0, -1, 1);
+        // z
+        const T ez = mulv(mulv(half, Wkp - Wkm), mad(hwd, Wkp + Wkm, Wc));
+        // x
+        const T um = mad(Z.w1(), Umkp, mulv(Z.w0(), Um)), du = uz - um, ws = Wm + Wc;
+        T g;
+        if constexpr (PROF) g = mad(qq, um, mad(pp, uz, R.u)); else g = mad(qq, um, mulv(pp, uz));
+        const T cx = mad(mulv(hwd, ws), du, mulv(mulv(half, W10 - Wm), g));
+        // y
+        const T vzm = mad(Z.w1(), Vjmkp, mulv(Z.w0(), Vjm)), wym = mad(Y.w1m(), Wc, mulv(Y.w0m(), Wjm));
+        const T m = mulv(qq, vzm + vz);
+        const T cy = nmad(wym, mad(wd, vzm, m), mulv(wy, mad(wd, vz, m)));
+        if constexpr (LES || WM) {
+            T nx1 = nu, ny1 = nu, nz1 = nu, nz2 = nu, fx2, fy2;
+            if constexpr (LES) {
+                const T n0 = N(0, 0, 0), np = N(0, 0, 1), z0 = Z.w0(), z1 = Z.w1(), nz = mad(z1, np, mulv(z0, n0));
+                nx1 = mad(half, mad(z1, N(-1, 0, 1), mad(z0, N(-1, 0, 0), nz)), nu);
+                if (in_lo) ny1 = mad(Y.w0m(), mad(z1, N(0, -1, 1), mulv(z0, N(0, -1, 0))), mad(Y.w1m(), nz, nu));
+                nz1 = nu + n0;
+                nz2 = nu + np;
+                fx2 = fxz;
+                fy2 = vrow ? fyz : mulv(nu, mad(Y.invf(), dWy, mulv(Z.invf(), dVz)));   // the top wall: nu_t does not reach it
+            } else {
+                fx2 = mulv(nu, mad(inv_dx, dWx, mulv(Z.invf(), dUz)));
+                fy2 = mulv(nu, mad(Y.invf(), dWy, mulv(Z.invf(), dVz)));
+            }
+            T fy1 = mulv(ny1, mad(Y.invfm(), Wc - Wjm, mulv(Z.invf(), Vjmkp - Vjm)));
+            if (wall_lo) fy1 = wall_flux<T>(tau_z + k * d.Nx + i);
+            if (wall_hi) fy2 = wall_flux<T>(tau_z + (d.Nz + k) * d.Nx + i);
+            const T fx1 = mulv(nx1, mad(inv_dx, Wc - Wm, mulv(Z.invf(), Umkp - Um)));
+            const T fz = nmad(nz1, mulv(Z.invc(), Wc - Wkm), mulv(nz2, mulv(Z.invcp(), Wkp - Wc)));
+            T r = mad(Z.invf(), mad(fz, T(2), -ez), bcast<T>(K.dPdz));
+            r = mad(inv_dx, (fx2 - fx1) - cx, r);
+            rw = mad(Y.invc(), (fy2 - fy1) - cy, r);
+        } else {
+            T F = nmad(Z.invc(), Wc - Wkm, mulv(Z.invcp(), Wkp - Wc));
+            T r = mad(Z.invf(), mad(bcast<T>(K.nu2), F, -ez), bcast<T>(K.dPdz));
+            F = mad(Z.invf(), dUz - (Umkp - Um), mulv(inv_dx, mad(m2, Wc, W10 + Wm)));
+            r = mad(inv_dx, mad(nu, F, -cx), r);
+            F = nmad(Y.invfm(), Wc - Wjm, mulv(Y.invf(), dWy));
+            F = mad(Z.invf(), dVz - (Vjmkp - Vjm), F);
+            rw = mad(Y.invc(), mad(nu, F, -cy), r);
+        }
     }
-    T dUkp = Ukp - Uc, dUkm = Uc - Ukm, dUip = Uip - Uc, dUim = Uc - Uim;
-    if constexpr (Fp32Forms<T>::value) {   // x and z differences of U from the deviations
-        T Udc = q.Ud(0, 0, 0);
-        dUkp = q.Ud(0, 0, 1) - Udc; dUkm = Udc - q.Ud(0, 0, -1);
-        dUip = q.Ud(1, 0, 0) - Udc; dUim = Udc - q.Ud(-1, 0, 0);
-    }
-    T tk = Z.divf(dUkp), tkm = Z.divfm(dUkm);
-    T fz2 = nu_z2 * (tk + (W10 - W00) * a.inv_dx);
-    T fz1 = nu_z1 * (tkm + (W1m - W0m) * a.inv_dx);
-    r = r + T(2) * a.inv_dx2 * (nu_x2 * dUip - nu_x1 * dUim) + inv_dy3 * (fy2 - fy1) + inv_dz3 * (fz2 - fz1) + a.dPdx;
-    return r;
 }
 
-template <typename T, bool LES, bool WM, typename Q, typename SA>
-__device__ __forceinline__ T rhs_v_at(const SA &a, const Q &q, const AxisLocal<T> &Y, const AxisLocal<T> &Z, int i, int j, int k) {
-    const Dims &d = a.d;
-    (void)i; (void)d;
-    T wa = a.w_adv, wd = T(1) - wa;
-    T Vc = q.V(0, 0, 0), Vjm = q.V(0, -1, 0), Vjp = q.V(0, 1, 0);
-    T Vim = q.V(-1, 0, 0), Vip = q.V(1, 0, 0), Vkm = q.V(0, 0, -1), Vkp = q.V(0, 0, 1);
-    // -d(vv)/dy
-    T t1 = T(0.5) * (Vc + Vjp), t0 = T(0.5) * (Vjm + Vc);
-    T r = -Y.divf(wd * (t1 * t1 - t0 * t0) + wa * Vc * (t1 - t0));
-    // -d(uv)/dx: u at y face j (weighted), v at x faces
-    T Uc = q.U(0, 0, 0), Um = q.U(-1, 0, 0), Ucp = q.U(0, 1, 0), Ump = q.U(-1, 1, 0);
-    {
-        T u1 = Y.w0() * Uc + Y.w1() * Ucp, u0 = Y.w0() * Um + Y.w1() * Ump;
-        T v1 = T(0.5) * (Vc + Vip), v0 = T(0.5) * (Vim + Vc);
-        if constexpr (Fp32Forms<T>::value) {   // u1 v1 - u0 v0 = u1 (v1 - v0) + v0 (u1 - u0), u1 - u0 from deviations
-            T du = Y.w0() * (q.Ud(0, 0, 0) - q.Ud(-1, 0, 0)) + Y.w1() * (q.Ud(0, 1, 0) - q.Ud(-1, 1, 0));
-            r = r - (wd * (u1 * (v1 - v0) + v0 * du) + wa * T(0.5) * (u0 + u1) * (v1 - v0)) * a.inv_dx;
-        } else {
-            r = r - (wd * (u1 * v1 - u0 * v0) + wa * T(0.5) * (u0 + u1) * (v1 - v0)) * a.inv_dx;
-        }
-    }
-    // -d(vw)/dz: v at z faces (weighted), w at y face j (weighted)
-    T Wc = q.W(0, 0, 0), Wjp = q.W(0, 1, 0), Wkm = q.W(0, 0, -1), Wkmjp = q.W(0, 1, -1);
-    {
-        T v1 = Z.w0() * Vc + Z.w1() * Vkp, v0 = Z.w0m() * Vkm + Z.w1m() * Vc;
-        T w1 = Y.w0() * Wc + Y.w1() * Wjp, w0 = Y.w0() * Wkm + Y.w1() * Wkmjp;
-        r = r - Z.divc(wd * (v1 * w1 - v0 * w0) + wa * T(0.5) * (w0 + w1) * (v1 - v0));
-    }
-    // viscous
-    T inv_dz3 = Z.invc();
-    T inv_dzg1 = Z.invfm(), inv_dzg2 = Z.invf();
-    T inv_dy1 = Y.invc(), inv_dy2 = Y.invcp(), inv_dy3 = Y.invf();
-    T two_inv_dy3 = T(2) * inv_dy3;
-    T nu = a.nu;
-    T nu_x1 = nu, nu_x2 = nu, nu_y1 = nu, nu_y2 = nu, nu_z1 = nu, nu_z2 = nu;
-    if (LES) {
-        T n_c = q.N(0, 0, 0), n_jp = q.N(0, 1, 0);
-        T w0 = Y.w0(), w1 = Y.w1();
-        nu_x1 = nu + T(0.5) * (w0 * q.N(-1, 0, 0) + w1 * q.N(-1, 1, 0) + w0 * n_c + w1 * n_jp);
-        nu_x2 = nu + T(0.5) * (w0 * n_c + w1 * n_jp + w0 * q.N(1, 0, 0) + w1 * q.N(1, 1, 0));
-        nu_y1 = nu + n_c;
-        nu_y2 = nu + n_jp;
-        nu_z1 = nu + Z.w0m() * (w0 * q.N(0, 0, -1) + w1 * q.N(0, 1, -1)) + Z.w1m() * (w0 * n_c + w1 * n_jp);
-        nu_z2 = nu + Z.w0() * (w0 * n_c + w1 * n_jp) + Z.w1() * (w0 * q.N(0, 0, 1) + w1 * q.N(0, 1, 1));
-    }
-    T fx2 = nu_x2 * ((Vip - Vc) * a.inv_dx + (Ucp - Uc) * inv_dy3);
-    T fx1 = nu_x1 * ((Vc - Vim) * a.inv_dx + (Ump - Um) * inv_dy3);
-    T fz2 = nu_z2 * ((Vkp - Vc) * inv_dzg2 + (Wjp - Wc) * inv_dy3);
-    T fz1 = nu_z1 * ((Vc - Vkm) * inv_dzg1 + (Wkmjp - Wkm) * inv_dy3);
-    r = r + a.inv_dx * (fx2 - fx1) + two_inv_dy3 * (nu_y2 * (Vjp - Vc) * inv_dy2 - nu_y1 * (Vc - Vjm) * inv_dy1) + inv_dz3 * (fz2 - fz1);
-    return r;
-}
-
-template <typename T, bool LES, bool WM, typename Q, typename SA>
-__device__ __forceinline__ T rhs_w_at(const SA &a, const Q &q, const AxisLocal<T> &Y, const AxisLocal<T> &Z,
-                                    const double *__restrict__ tau_z, int i, int j, int k) {
-    const Dims &d = a.d;
-    bool wm_band = WM && a.wm && (j + 2 <= 1 + a.nwl || j + 2 >= d.Ny + 2 - a.nwl);
-    T wa = wm_band ? T(0) : a.w_adv, wd = T(1) - wa;
-    T Wc = q.W(0, 0, 0), Wkm = q.W(0, 0, -1), Wkp = q.W(0, 0, 1);
-    T Wim = q.W(-1, 0, 0), Wip = q.W(1, 0, 0), Wjm = q.W(0, -1, 0), Wjp = q.W(0, 1, 0);
-    // -d(ww)/dz
-    T t1 = T(0.5) * (Wc + Wkp), t0 = T(0.5) * (Wkm + Wc);
-    T r = -Z.divf(wd * (t1 * t1 - t0 * t0) + wa * Wc * (t1 - t0));
-    // -d(uw)/dx: u at z face k (weighted), w at x faces
-    T Uc = q.U(0, 0, 0), Um = q.U(-1, 0, 0), Ukp = q.U(0, 0, 1), Umkp = q.U(-1, 0, 1);
-    {
-        T u1 = Z.w0() * Uc + Z.w1() * Ukp, u0 = Z.w0() * Um + Z.w1() * Umkp;
-        T w1 = T(0.5) * (Wc + Wip), w0 = T(0.5) * (Wim + Wc);
-        if constexpr (Fp32Forms<T>::value) {   // u1 w1 - u0 w0 = u1 (w1 - w0) + w0 (u1 - u0), u1 - u0 from deviations
-            T du = Z.w0() * (q.Ud(0, 0, 0) - q.Ud(-1, 0, 0)) + Z.w1() * (q.Ud(0, 0, 1) - q.Ud(-1, 0, 1));
-            r = r - (wd * (u1 * (w1 - w0) + w0 * du) + wa * T(0.5) * (u0 + u1) * (w1 - w0)) * a.inv_dx;
-        } else {
-            r = r - (wd * (u1 * w1 - u0 * w0) + wa * T(0.5) * (u0 + u1) * (w1 - w0)) * a.inv_dx;
-        }
-    }
-    // -d(vw)/dy: v at z face k (weighted), w at y faces (weighted)
-    T Vc = q.V(0, 0, 0), Vkp = q.V(0, 0, 1), Vjm = q.V(0, -1, 0), Vjmkp = q.V(0, -1, 1);
-    {
-        T v1 = Z.w0() * Vc + Z.w1() * Vkp, v0 = Z.w0() * Vjm + Z.w1() * Vjmkp;
-        T w1 = Y.w0() * Wc + Y.w1() * Wjp, w0 = Y.w0m() * Wjm + Y.w1m() * Wc;
-        r = r - Y.divc(wd * (v1 * w1 - v0 * w0) + wa * T(0.5) * (v0 + v1) * (w1 - w0));
-    }
-    // viscous
-    T inv_dz1 = Z.invc(), inv_dz2 = Z.invcp(), inv_dz3 = Z.invf();
-    T two_inv_dz3 = T(2) * inv_dz3;
-    T inv_dy3 = Y.invc();
-    T nu = a.nu;
-    T nu_x1 = nu, nu_x2 = nu, nu_y1 = nu, nu_y2 = nu, nu_z1 = nu, nu_z2 = nu;
-    if (LES) {
-        T n_c = q.N(0, 0, 0), n_kp = q.N(0, 0, 1);
-        T z0 = Z.w0(), z1 = Z.w1();
-        nu_x1 = nu + T(0.5) * (z0 * (n_c + q.N(-1, 0, 0)) + z1 * (n_kp + q.N(-1, 0, 1)));
-        nu_x2 = nu + T(0.5) * (z0 * (n_c + q.N(1, 0, 0)) + z1 * (n_kp + q.N(1, 0, 1)));
-        if (!(d.yper == 0 && j == 0))
-            nu_y1 = nu + z0 * (Y.w0m() * q.N(0, -1, 0) + Y.w1m() * n_c) + z1 * (Y.w0m() * q.N(0, -1, 1) + Y.w1m() * n_kp);
-        if (!(d.yper == 0 && j == d.Ny - 1))
-            nu_y2 = nu + z0 * (Y.w0() * n_c + Y.w1() * q.N(0, 1, 0)) + z1 * (Y.w0() * n_kp + Y.w1() * q.N(0, 1, 1));
-        nu_z1 = nu + n_c;
-        nu_z2 = nu + n_kp;
-    }
-    T tj = Y.divf(Wjp - Wc), tjm = Y.divfm(Wc - Wjm);
-    T fy2 = nu_y2 * (tj + (Vkp - Vc) * inv_dz3);
-    T fy1 = nu_y1 * (tjm + (Vjmkp - Vjm) * inv_dz3);
-    if (WM && a.wm) {
-        if (j == 0) fy1 = wall_flux<T>(tau_z + k * d.Nx + i);
-        if (j == d.Ny - 1) fy2 = wall_flux<T>(tau_z + (d.Nz + k) * d.Nx + i);
-    }
-    T fx2 = nu_x2 * ((Wip - Wc) * a.inv_dx + (Ukp - Uc) * inv_dz3);
-    T fx1 = nu_x1 * ((Wc - Wim) * a.inv_dx + (Umkp - Um) * inv_dz3);
-    r = r + a.inv_dx * (fx2 - fx1) + inv_dy3 * (fy2 - fy1) +
-        two_inv_dz3 * (nu_z2 * (Wkp - Wc) * inv_dz2 - nu_z1 * (Wc - Wkm) * inv_dz1) + a.dPdz;
-    return r;
+// wd of row j: 1 in the wall band of the wall model, else the blend's
+template <typename T, bool WM, typename SA> __device__ __forceinline__ T row_wd(const SA &a, int j) {
+    if (WM && a.wm && (j < a.nwl || j >= a.d.Ny - a.nwl)) return T(1);
+    return bcast<T>(a.rc.wd);
 }
 
 // Stage coefficients of the Butcher-form RK3 update (src/time_integration.f90:255-259, :393-397, :525-532):
@@ -519,12 +556,10 @@ template <typename T, int PX> struct TileQ {
 template <int PX> struct TileQ2 {
     const float *u[3], *v[3], *w[3], *n[3];
     int c;
-    F2 ub[3];
     static __device__ __forceinline__ F2 ld(const float *pl, int off) {
         if ((off & 1) == 0) return F2(*reinterpret_cast<const float2 *>(pl + off));
         return F2::pair(pl[off], pl[off + 1]);
     }
-    __device__ __forceinline__ F2 U(int di, int dj, int dk) const { return ld(u[dk + 1] + c, dj * PX + di) + ub[dj + 1]; }
     __device__ __forceinline__ F2 Ud(int di, int dj, int dk) const { return ld(u[dk + 1] + c, dj * PX + di); }
     __device__ __forceinline__ F2 V(int di, int dj, int dk) const { return ld(v[dk + 1] + c, dj * PX + di); }
     __device__ __forceinline__ F2 W(int di, int dj, int dk) const { return ld(w[dk + 1] + c, dj * PX + di); }
@@ -537,7 +572,7 @@ template <int PX> struct TileQ2 {
 // update (or, with rhs_only, the right-hand sides themselves).  Shared by the one-cell stage kernels.
 template <typename T, bool LES, bool WM, bool HYB, typename Q>
 __device__ __forceinline__ void stage_cell(const StepArgs<T> &a, const Q &q, const AxisLocal<T> &Y,
-                                           const double *__restrict__ tau_x, const double *__restrict__ tau_z,
+                                           const RowProfile<T> &R, const double *__restrict__ tau_x, const double *__restrict__ tau_z,
                                            const StageCoef &sc, int i, int j, int k, T *__restrict__ uo,
                                            T *__restrict__ vo, T *__restrict__ wo, T *__restrict__ f1u,
                                            T *__restrict__ f1v, T *__restrict__ f1w, T *__restrict__ us,
@@ -554,9 +589,8 @@ __device__ __forceinline__ void stage_cell(const StepArgs<T> &a, const Q &q, con
     }
     AxisLocal<T> Z;
     Z.load(a.mz, k);
-    T ru = rhs_u_at<T, LES, WM>(a, q, Y, Z, tau_x, i, j, k);
-    T rw = rhs_w_at<T, LES, WM>(a, q, Y, Z, tau_z, i, j, k);
-    T rv = vrow ? rhs_v_at<T, LES, WM>(a, q, Y, Z, i, j, k) : T(0);
+    T ru, rv, rw;
+    rhs_at<T, LES, WM>(a, q, Y, R, Z, tau_x, tau_z, i, j, k, vrow, ru, rv, rw);
     if constexpr (HYB) {
         ru = ru + a.adv[p]; rw = rw + a.adv[2 * d.cells + p];
         if (vrow) rv = rv + a.adv[d.cells + p];
@@ -591,8 +625,7 @@ __device__ __forceinline__ void stage_cell(const StepArgs<T> &a, const Q &q, con
 // rules (no-slip mirror of U and W, zero V and nu_t on the ghost rows).  Every thread then evaluates the three
 // right-hand sides of its cell from shared memory and writes the RK3 update (or, with rhs_only, the right-hand
 // sides themselves for the unit entry point; with KIND 1, nu_t).
-// WM = false compiles the flat-wall model out; with WM = true the runtime flag StepArgs::wm decides (the FP64 form
-// always takes that variant: without the branches its register allocation spills).
+// WM = false compiles the flat-wall model out.
 // CORR (stages 2 and 3 of a step whose stage kernel is the only reader of the corrected velocity): U, V, W are the
 // previous stage's u*, and the loader applies that stage's projection, u = u* - grad(phi) with StepArgs::phi, to
 // every plane element it copies, before the wall rules -- the arithmetic of k_correct, so the values are the ones
@@ -730,6 +763,8 @@ __device__ __forceinline__ void k_tiled_body(const BC &bc, const StepArgs<T> &a,
 
     AxisLocal<T> Y;   // this thread's y metrics (FP32: read here once for every plane)
     Y.load(a.my, min(j, Ny - 1));
+    RowProfile<T> R;
+    R.load(ubr, Y, row_wd<T, WM>(a, j));
 
     // planes k0-1, k0, k0+1 into slots 0, 1, 2; plane k lives in slot (k - k0 + 1) & 3 (CORR: phi k0-1 .. k0+2)
     issue(0, k0 - 1); issue(1, k0); issue(2, k0 + 1);
@@ -758,7 +793,7 @@ __device__ __forceinline__ void k_tiled_body(const BC &bc, const StepArgs<T> &a,
             if (KIND == 1) {
                 nut_out[p] = nut_at<T>(a, q, i, j, k);
             } else {
-                stage_cell<T, LES, WM, KIND == 2>(a, q, Y, tau_x, tau_z, sc, i, j, k, uo, vo, wo, f1u, f1v, f1w, us, vs,
+                stage_cell<T, LES, WM, KIND == 2>(a, q, Y, R, tau_x, tau_z, sc, i, j, k, uo, vo, wo, f1u, f1v, f1w, us, vs,
                                                   wsf, rhs_only);
             }
         }
@@ -781,11 +816,11 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_tiled(StepAr
 
 
 // One thread's pair of cells (i, i+1) of plane k from the shared-memory neighbourhood q: the three right-hand sides
-// and the RK3 stage update (or, with rhs_only, the right-hand sides themselves).  zm holds the eight z metrics of
-// plane k (AxisLocal<F2>::load8 order).  Shared by the packed stage kernels.
+// and the RK3 stage update (or, with rhs_only, the right-hand sides themselves).  zm holds the z metrics of
+// plane k (AxisLocal<F2>::load_pairs order).  Shared by the packed stage kernels.
 template <bool LES, bool WM, bool HYB, int PX>
 __device__ __forceinline__ void stage_pair(const StepArgs<float> &a, const TileQ2<PX> &q, const AxisLocal<F2> &Y,
-                                           const float *zm, const double *__restrict__ tau_x,
+                                           const RowProfile<F2> &R, const float *zm, const double *__restrict__ tau_x,
                                            const double *__restrict__ tau_z, const StageCoef &sc, int i, int j, int k,
                                            float *__restrict__ uo, float *__restrict__ vo, float *__restrict__ wo,
                                            float *__restrict__ f1u, float *__restrict__ f1v, float *__restrict__ f1w,
@@ -804,10 +839,9 @@ __device__ __forceinline__ void stage_pair(const StepArgs<float> &a, const TileQ
         if (vrow) fv = ld2(f1v);
     }
     AxisLocal<F2> Z;
-    Z.load8(zm);
-    F2 ru = rhs_u_at<F2, LES, WM>(a, q, Y, Z, tau_x, i, j, k);
-    F2 rw = rhs_w_at<F2, LES, WM>(a, q, Y, Z, tau_z, i, j, k);
-    F2 rv = vrow ? rhs_v_at<F2, LES, WM>(a, q, Y, Z, i, j, k) : F2(0.0f);
+    Z.load_pairs(zm);
+    F2 ru, rv, rw;
+    rhs_at<F2, LES, WM>(a, q, Y, R, Z, tau_x, tau_z, i, j, k, vrow, ru, rv, rw);
     if constexpr (HYB) {
         ru = ru + ld2(a.adv); rw = rw + ld2(a.adv + 2 * d.cells);
         if (vrow) rv = rv + ld2(a.adv + d.cells);
@@ -855,9 +889,9 @@ __device__ __forceinline__ void k_tiled2_body(const BC &bc, const StepArgs<float
     // CORR phi tile: two more columns (an even pitch keeps pairs aligned) and one more row
     constexpr int PXP = PX + 2, PSP2 = PXP * (PY + 1) / 2, PERP = (PSP2 + NT - 1) / NT;
     __shared__ __align__(16) float smp[CORR ? 5 : 1][CORR ? 2 * PSP2 : 2];
-    // the z metrics of planes k .. k+2 (AxisLocal<F2>::load8 order), copied with the planes: under the streaming
+    // the z metrics of planes k .. k+2 (AxisLocal<F2>::load_pairs order), copied with the planes: under the streaming
     // tile copies the metric tables do not stay in L1, and every thread needs them at the start of its plane
-    __shared__ float zmr[4][8];
+    __shared__ __align__(16) float zmr[4][ZPAIRS];
     const Dims &d = a.d;
     const int Nx = d.Nx, Ny = d.Ny, Nz = d.Nz;
     const int i0 = bc.idx().x * TXC, j0 = bc.idx().y * TY;
@@ -922,7 +956,7 @@ __device__ __forceinline__ void k_tiled2_body(const BC &bc, const StepArgs<float
         }
     };
     auto issue_z = [&](int k) {   // the z metrics of plane k (k0 <= k < kend) into zmr[(k - k0) & 3]
-        if (threadIdx.x < 8) cp_async<4>(&zmr[(k - k0) & 3][threadIdx.x], AxisLocal<F2>::metric_src(a.mz, k, threadIdx.x));
+        if (threadIdx.x < ZPAIRS / 2) cp_async<8>(&zmr[(k - k0) & 3][2 * threadIdx.x], a.zm8 + ZPAIRS * k + 2 * threadIdx.x);
     };
     auto issue = [&](int slot, int k) {
         int kw = k < 0 ? k + Nz : (k >= Nz ? k - Nz : k);
@@ -988,6 +1022,8 @@ __device__ __forceinline__ void k_tiled2_body(const BC &bc, const StepArgs<float
     }
     AxisLocal<F2> Y;
     Y.load(a.my, min(j, Ny - 1));
+    RowProfile<F2> R;
+    R.load(ubr, Y, row_wd<F2, WM>(a, j));
 
     issue(0, k0 - 1); issue(1, k0); issue(2, k0 + 1);
     issue_phi(k0 - 1); issue_phi(k0); issue_phi(k0 + 1); issue_phi(k0 + 2); issue_phi(k0 + 3);
@@ -1009,12 +1045,11 @@ __device__ __forceinline__ void k_tiled2_body(const BC &bc, const StepArgs<float
         if (active) {
             TileQ2<PX> q;
             q.c = cloc;
-            q.ub[0] = ubr[0]; q.ub[1] = ubr[1]; q.ub[2] = ubr[2];
             q.u[0] = sm[0][sm_]; q.u[1] = sm[0][s0]; q.u[2] = sm[0][sp];
             q.v[0] = sm[1][sm_]; q.v[1] = sm[1][s0]; q.v[2] = sm[1][sp];
             q.w[0] = sm[2][sm_]; q.w[1] = sm[2][s0]; q.w[2] = sm[2][sp];
             q.n[0] = sm[NF - 1][sm_]; q.n[1] = sm[NF - 1][s0]; q.n[2] = sm[NF - 1][sp];
-            stage_pair<LES, WM, HYB>(a, q, Y, zmr[(k - k0) & 3], tau_x, tau_z, sc, i, j, k, uo, vo, wo, f1u, f1v, f1w,
+            stage_pair<LES, WM, HYB>(a, q, Y, R, zmr[(k - k0) & 3], tau_x, tau_z, sc, i, j, k, uo, vo, wo, f1u, f1v, f1w,
                                      us, vs, wsf, rhs_only);
         }
         cp_async_wait_all();

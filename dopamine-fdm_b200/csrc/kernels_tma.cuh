@@ -89,7 +89,7 @@ template <bool LES, bool CORR> struct TmaSmem {
     alignas(128) unsigned char p[CORR ? tma::SLOTS : 1][CORR ? tma::PSLOT : 128];
     alignas(128) unsigned char pp[CORR ? tma::SLOTS : 1][2][CORR ? tma::QSLOT : 128];
     alignas(8) uint64_t full[tma::SLOTS];
-    alignas(16) float zm[tma::SLOTS][8];   // the z metrics of each slot's plane (32-byte bulk copies)
+    alignas(16) float zm[tma::SLOTS][ZPAIRS];   // the z metrics of each slot's plane (64-byte bulk copies)
 };
 
 template <bool LES, bool WM, bool HYB, bool CORR>
@@ -120,9 +120,9 @@ __global__ void __launch_bounds__(256, 2) k_tma2(StepArgs<float> a, const __grid
     const bool edge = wrapl || wrapr || lo_row || hi_row;
     const int npatch = (wrapl ? 1 : 0) + (wrapr ? 1 : 0);
     // bytes one plane brings: every field's main box and its patches, (CORR) phi of the same plane, and the plane's
-    // eight z metrics
+    // z metrics
     const unsigned tx_bytes = NF * (BX * BY * 4 + npatch * PW * BY * 4) +
-                              (CORR ? BX * BYP * 4 + npatch * PW * BYP * 4 : 0) + 32;
+                              (CORR ? BX * BYP * 4 + npatch * PW * BYP * 4 : 0) + ZPAIRS * 4;
     // planes k0-1 .. kend are evaluated or read as neighbours; CORR also needs phi(kend+1) for the fix of kend
     const int plast = kend + (CORR ? 1 : 0);
 
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(256, 2) k_tma2(StepArgs<float> a, const __grid
             if (wrapl) load_box(S.pp[s][0], &tm.phip, Nx - 4, j0 - 1, pw, bar);
             if (wrapr) load_box(S.pp[s][1], &tm.phip, 0, j0 - 1, pw, bar);
         }
-        load_bulk(S.zm[s], a.zm8 + 8 * pw, 32, bar);
+        load_bulk(S.zm[s], a.zm8 + ZPAIRS * pw, ZPAIRS * 4, bar);
     };
     bool ok = true;
     auto wait_plane = [&](int p) {
@@ -237,6 +237,8 @@ __global__ void __launch_bounds__(256, 2) k_tma2(StepArgs<float> a, const __grid
     }
     AxisLocal<F2> Y;
     Y.load(a.my, min(j, Ny - 1));
+    RowProfile<F2> R;
+    R.load(ubr, Y, row_wd<F2, WM>(a, j));
 
     // planes k0-1, k0, k0+1 fixed before the first evaluation (CORR: their fix reads phi up to plane k0+2)
     for (int p = k0 - 1; p <= k0 + (CORR ? 2 : 1); ++p) wait_plane(p);
@@ -250,13 +252,12 @@ __global__ void __launch_bounds__(256, 2) k_tma2(StepArgs<float> a, const __grid
             const int sm_ = slot_of(k - 1), s0 = slot_of(k), sp = slot_of(k + 1);
             TileQ2<PX> q;
             q.c = cloc;
-            q.ub[0] = ubr[0]; q.ub[1] = ubr[1]; q.ub[2] = ubr[2];
             q.u[0] = (const float *)S.f[0][sm_]; q.u[1] = (const float *)S.f[0][s0]; q.u[2] = (const float *)S.f[0][sp];
             q.v[0] = (const float *)S.f[1][sm_]; q.v[1] = (const float *)S.f[1][s0]; q.v[2] = (const float *)S.f[1][sp];
             q.w[0] = (const float *)S.f[2][sm_]; q.w[1] = (const float *)S.f[2][s0]; q.w[2] = (const float *)S.f[2][sp];
             q.n[0] = (const float *)S.f[NF - 1][sm_]; q.n[1] = (const float *)S.f[NF - 1][s0];
             q.n[2] = (const float *)S.f[NF - 1][sp];
-            stage_pair<LES, WM, HYB>(a, q, Y, S.zm[s0], tau_x, tau_z, sc, i, j, k, uo, vo, wo, f1u, f1v, f1w, us, vs,
+            stage_pair<LES, WM, HYB>(a, q, Y, R, S.zm[s0], tau_x, tau_z, sc, i, j, k, uo, vo, wo, f1u, f1v, f1w, us, vs,
                                      wsf, rhs_only);
         }
         if (k + 2 <= kend) {
