@@ -181,8 +181,9 @@ struct dfdm_ctx {
     // with y and z exchanged (Ny = nz - 1 wall-bounded cells, Nz = ny - 2 periodic rows) so that the channel's
     // transforms and y solve serve it
     bool zwall = false;
-    int lx2 = 1, lxi2 = 1, thr_z2 = 256, thr_y2 = 256;   // x lines per block: forward, inverse
-    size_t smem_x2 = 0, smem_xi2 = 0, smem_z2 = 0, smem_y2 = 0;
+    int nsm = 148;                              // SMs of the device
+    int lx2 = 1, thr_x2 = 256, thr_z2 = 256, thr_y2 = 256;   // x lines per block; threads per block
+    size_t smem_x2 = 0, smem_z2 = 0, smem_y2 = 0;
     cudaStream_t own_stream = nullptr, stream = nullptr;
     // asynchronous state transfer (dfdm_set_state_async / dfdm_get_state_async): one copy stream per direction, one
     // FP64 staging buffer per field and direction, and events that keep a buffer from being refilled before its
@@ -393,6 +394,19 @@ int choose_kc(const Dims &d, int blocks_per_sm, int nsm, int tx = TILE_X, int ty
 }
 
 int reduce_grid(const Dims &d);
+// The row transforms of half-length M run lx N2 threads on lx lines per block, one step-1 item each: 256 threads, or by
+// halves down to one warp until the lines make at least three blocks for every SM, so that a small grid's lines spread over
+// the whole GPU.  Blocks of 256 threads on 24 to 64 lines took 6.6 (forward) and 4.8 us (inverse) at 64^3 cells against 4.5
+// and 4.1 us; two, three and five blocks per SM measured the same, and one per SM in a group, whose branches overlap (16
+// cases of 32^3 136.5 us per step against 139.7 with two).
+template <int M> int row_lines(long long lines, int nsm, int per_sm = 3) {
+    int lx = 256 / Split<M>::N2;
+    while (lx * Split<M>::N2 > 32 && (lines + lx - 1) / lx < (long long)per_sm * nsm) lx /= 2;
+    return lx;
+}
+template <typename T, int M> constexpr size_t row_smem(int lx) {
+    return (size_t)lx * RowLayout<M>::LD * sizeof(typename cplx_t<T>::type);
+}
 // blocks of a column transform of `nl` columns each: the (j, kx) columns of the z transforms (families 3, 5) or the
 // (kz, kx) columns of the periodic-y solve (family 4)
 int col_blocks(const Dims &d, int which, int nl) { return (d.Nxc * (which == 4 ? d.Nz : d.Ny) + nl - 1) / nl; }
@@ -407,7 +421,9 @@ template <typename T> struct Impl {
 
     static int setup_fft2l(dfdm_ctx *c) {
         const Dims &d = c->d;
-        int rc = DFDM_OK;
+        int rc = DFDM_OK, dev = 0;
+        CK(cudaGetDevice(&dev));
+        CK(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, dev));
         auto setattr = [&](const void *fn, size_t bytes) {
             if (rc) return;
             cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -415,14 +431,13 @@ template <typename T> struct Impl {
         };
         c->x2 = with_fft2l(d.Nx / 2, [&](auto n) {
             constexpr int N = decltype(n)::value;
-            const size_t perline = (size_t)(RowLayout<N>::LDA + RowLayout<N>::LDT) * sizeof(C);
-            c->lx2 = RowLines<T, N>::value;   // the forward kernel's loop bound assumes exactly this
-            c->smem_x2 = (size_t)c->lx2 * perline;
-            c->lxi2 = (int)std::max<size_t>(1, std::min<size_t>(64, 73728 / perline));   // measured best for the inverse
-            c->smem_xi2 = (size_t)c->lxi2 * RowLayout<N>::LDT * sizeof(C);
-            setattr((const void *)k_fwd_x2<T, true, N>, c->smem_x2);
-            setattr((const void *)k_fwd_x2<T, false, N>, c->smem_x2);
-            setattr((const void *)k_inv_x2<T, N>, c->smem_xi2);
+            c->lx2 = row_lines<N>((long long)d.Ny * d.Nz, c->nsm);
+            c->thr_x2 = c->lx2 * Split<N>::N2;
+            c->smem_x2 = row_smem<T, N>(c->lx2);
+            const size_t cap = row_smem<T, N>(256 / Split<N>::N2);   // of every grid with this row length
+            setattr((const void *)k_fwd_x2<T, true, N>, cap);
+            setattr((const void *)k_fwd_x2<T, false, N>, cap);
+            setattr((const void *)k_inv_x2<T, N>, cap);
         });
         c->z2 = with_fft2l(d.Nz, [&](auto n) {
             constexpr int N = decltype(n)::value;
@@ -450,10 +465,10 @@ template <typename T> struct Impl {
             with_fft2l(d.Nx / 2, [&](auto n) {
                 constexpr int N = decltype(n)::value;
                 if (from_div)
-                    k_fwd_x2<T, true, N><<<nb, 256, c->smem_x2, st>>>(poisson_args<T>(c), c->lx2, f(c->us), f(c->vs), f(c->wsf),
+                    k_fwd_x2<T, true, N><<<nb, c->thr_x2, c->smem_x2, st>>>(poisson_args<T>(c), c->lx2, f(c->us), f(c->vs), f(c->wsf),
                                                                        nullptr, (C *)c->spec, (const C *)c->tw_x, (const C *)c->twr_x);
                 else
-                    k_fwd_x2<T, false, N><<<nb, 256, c->smem_x2, st>>>(poisson_args<T>(c), c->lx2, nullptr, nullptr, nullptr,
+                    k_fwd_x2<T, false, N><<<nb, c->thr_x2, c->smem_x2, st>>>(poisson_args<T>(c), c->lx2, nullptr, nullptr, nullptr,
                                                                         src, (C *)c->spec, (const C *)c->tw_x, (const C *)c->twr_x);
             });
         } else {
@@ -991,10 +1006,10 @@ template <typename T> struct Impl {
         case 6: {   // inverse x
             long long lines = (long long)d.Ny * d.Nz;
             if (c->x2) {
-                int nb = (int)((lines + c->lxi2 - 1) / c->lxi2);
+                int nb = (int)((lines + c->lx2 - 1) / c->lx2);
                 with_fft2l(d.Nx / 2, [&](auto n) {
                     constexpr int N = decltype(n)::value;
-                    k_inv_x2<T, N><<<nb, 256, c->smem_xi2, st>>>(poisson_args<T>(c), c->lxi2, (const C *)c->spec, f(c->phi),
+                    k_inv_x2<T, N><<<nb, c->thr_x2, c->smem_x2, st>>>(poisson_args<T>(c), c->lx2, (const C *)c->spec, f(c->phi),
                                                                   (const C *)c->tw_x, (const C *)c->twr_x);
                 });
             } else {
@@ -3101,21 +3116,31 @@ int members_step_enqueue(const std::vector<dfdm_ctx *> &cs, cudaStream_t st,
             if ((rc = launch_stage_jobs(stage[v], v, corr, walk, walk_cap, st))) return rc;
         // ---- div u* + forward x, per length ----
         std::map<int, std::vector<FwdXJob>> fx;
-        std::map<int, size_t> fx_smem;
+        // lines per block from those of the whole branch (one row length), which share the GPU
+        long long lines_all = 0;
+        int lx = 1, xthr = 256;
+        size_t xsmem = 0;
+        for (dfdm_ctx *c : cs) lines_all += (long long)c->d.Ny * c->d.Nz;
+        with_fft2l(cs[0]->d.Nx / 2, [&](auto n) {
+            constexpr int M = decltype(n)::value;
+            lx = row_lines<M>(lines_all, cs[0]->nsm, 1);
+            xthr = lx * Split<M>::N2;
+            xsmem = row_smem<float, M>(lx);
+        });
         for (dfdm_ctx *c : cs) {
             FwdXJob J;
             const long long lines = (long long)c->d.Ny * c->d.Nz;
-            J.grid = dim3((unsigned)((lines + c->lx2 - 1) / c->lx2), 1, 1);
-            J.a = poisson_args<float>(c); J.lx = c->lx2;
+            J.lx = lx;
+            J.grid = dim3((unsigned)((lines + J.lx - 1) / J.lx), 1, 1);
+            J.a = poisson_args<float>(c);
             J.U = (const float *)c->us; J.V = (const float *)c->vs; J.W = (const float *)c->wsf; J.src = nullptr;
             J.spec = (C *)c->spec; J.tw = (const C *)c->tw_x; J.twr = (const C *)c->twr_x;
             fx[c->d.Nx / 2].push_back(J);
-            fx_smem[c->d.Nx / 2] = c->smem_x2;
         }
         for (auto &kv : fx) {
             with_fft2l(kv.first, [&](auto n) {
                 constexpr int M = decltype(n)::value;
-                rc = launch_groups(kv.second, [&](const GroupTable<FwdXJob> &t, int nb) { kg_fwd_x<M><<<nb, 256, fx_smem[M], st>>>(t); });
+                rc = launch_groups(kv.second, [&](const GroupTable<FwdXJob> &t, int nb) { kg_fwd_x<M><<<nb, xthr, xsmem, st>>>(t); });
             });
             if (rc) return rc;
         }
@@ -3165,20 +3190,19 @@ int members_step_enqueue(const std::vector<dfdm_ctx *> &cs, cudaStream_t st,
         if ((rc = col_family(1))) return rc;
         // ---- inverse x, per length ----
         std::map<int, std::vector<InvXJob>> ix;
-        std::map<int, size_t> ix_smem;
         for (dfdm_ctx *c : cs) {
             InvXJob J;
             const long long lines = (long long)c->d.Ny * c->d.Nz;
-            J.grid = dim3((unsigned)((lines + c->lxi2 - 1) / c->lxi2), 1, 1);
-            J.a = poisson_args<float>(c); J.lx = c->lxi2;
+            J.lx = lx;
+            J.grid = dim3((unsigned)((lines + J.lx - 1) / J.lx), 1, 1);
+            J.a = poisson_args<float>(c);
             J.spec = (const C *)c->spec; J.phi = (float *)c->phi; J.tw = (const C *)c->tw_x; J.twr = (const C *)c->twr_x;
             ix[c->d.Nx / 2].push_back(J);
-            ix_smem[c->d.Nx / 2] = c->smem_xi2;
         }
         for (auto &kv : ix) {
             with_fft2l(kv.first, [&](auto n) {
                 constexpr int M = decltype(n)::value;
-                rc = launch_groups(kv.second, [&](const GroupTable<InvXJob> &t, int nb) { kg_inv_x<M><<<nb, 256, ix_smem[M], st>>>(t); });
+                rc = launch_groups(kv.second, [&](const GroupTable<InvXJob> &t, int nb) { kg_inv_x<M><<<nb, xthr, xsmem, st>>>(t); });
             });
             if (rc) return rc;
         }
@@ -3396,8 +3420,8 @@ int group_attributes(dfdm_group *g) {
     for (dfdm_ctx *c : g->cs) {
         with_fft2l(c->d.Nx / 2, [&](auto n) {
             constexpr int M = decltype(n)::value;
-            setattr((const void *)kg_fwd_x<M>, c->smem_x2);
-            setattr((const void *)kg_inv_x<M>, c->smem_xi2);
+            setattr((const void *)kg_fwd_x<M>, row_smem<float, M>(256 / Split<M>::N2));
+            setattr((const void *)kg_inv_x<M>, row_smem<float, M>(256 / Split<M>::N2));
         });
         with_fft2l(c->d.Nz, [&](auto n) {
             constexpr int L = decltype(n)::value;

@@ -113,24 +113,17 @@ template <typename F> inline bool with_fft2l(int n, F &&f) {
     return false;
 }
 
-// Shared-memory row layouts of the row transforms (x lines), in complex elements:
-//   LDA: stride of natural-order lines (padded to 8 mod 16 so two lines in one half-warp use disjoint banks)
-//   LDT: stride of the step-1 output lines, element k1*N2 + n2 at k1*(N2+1) + n2
+// Shared memory of the row transforms (x lines), in complex elements: line ll at ll * LD, holding either the line in
+// natural order or the step-1 outputs, element k1*N2 + n2 at k1*(N2+1) + n2.  LD is 8 mod 16, so that two lines in one
+// half-warp use disjoint banks.
 template <int N> struct RowLayout {
     static constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
     static constexpr int pad8(int x) { return x + ((8 - (x % 16) + 16) % 16); }
-    static constexpr int LDA = pad8(N);
-    static constexpr int LDT = pad8(N1 * (N2 + 1));
-};
-
-// x lines per block of the row transforms: as many as fit in 56 KB of shared memory (4 blocks of 256 threads per SM)
-template <typename T, int N> struct RowLines {
-    static constexpr int bytes = (RowLayout<N>::LDA + RowLayout<N>::LDT) * 2 * (int)sizeof(T);
-    static constexpr int value = (57344 / bytes) < 1 ? 1 : ((57344 / bytes) > 64 ? 64 : (57344 / bytes));
+    static constexpr int LD = pad8(N1 * (N2 + 1));
 };
 
 // Step 1 of a row transform for one (line, n2) item: v holds x[n1*N2 + n2], n1 = 0..N1-1, on entry; the twiddled
-// step-1 outputs go to t (layout LDT).
+// step-1 outputs go to tl (RowLayout).
 template <typename T, bool INV, int N>
 __device__ __forceinline__ void row_step1(typename cplx_t<T>::type *v, typename cplx_t<T>::type *tl, int n2,
                                           const typename cplx_t<T>::type *__restrict__ tw) {

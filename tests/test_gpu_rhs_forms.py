@@ -1,6 +1,7 @@
 """The right-hand sides of every form the stage kernels are compiled in (DNS, eddy viscosity, wall model; skew-symmetric and
 divergence form, with and without the wall band; periodic and wall-bounded y) on a grid with partial tiles in x and y, and
 the wall model on column counts around a block's, against the oracle: FP64 1e-12, FP32 1e-5 relative L2."""
+import numpy as np
 import pytest
 
 from conftest import interior, rel_l2
@@ -10,12 +11,22 @@ from dfdm.native import Solver
 pytestmark = pytest.mark.gpu
 
 
-def _case(wall, sgs, wm, scheme, nwl=-1, nx=68, nz=14, filt=-1):
+def _case(wall, sgs, wm, scheme, nwl=-1, nx=62, nz=14, filt=-1):
     if not wall:
         return cases.tgv(16, Re=400.0, name="box").with_(nx=nx, ny=14, nz=nz, sgs_model=sgs, advection_scheme=scheme)
     return cases.Case(name="walls", nx=nx, ny=12, nz=nz, Lx_i=4.0, Ly_i=2.0, Lz_i=1.5, grid_type=2, alpha_grid=2.0, nu=2e-3,
                       dt=1e-3, dPdx=1.0, sgs_model=sgs, flat_wall_model_flag=wm, advection_scheme=scheme,
                       adv_wall_layers=nwl, wm_filter_mode=filt, ic="reichardt_gauss", ic_amplitude=1.0, noise=0.25, seed=5)
+
+
+def _state(c):
+    """The case's mean with noise of a quarter of its amplitude on every component (no component small by symmetry)."""
+    U, V, W, P = cases.initial_condition(c)
+    rng = np.random.default_rng(9)
+    for a in (U, V, W):
+        a += rng.normal(0.0, 0.25, size=a.shape)
+    cases.fill_ghosts(c, U, V, W)
+    return U, V, W, P
 
 
 FORMS = [(wall, sgs, wm, scheme, nwl) for wall in (True, False) for sgs in (0, 2) for wm in (0, 1) for scheme in (0, 1)
@@ -25,7 +36,7 @@ FORMS = [(wall, sgs, wm, scheme, nwl) for wall in (True, False) for sgs in (0, 2
 @pytest.mark.parametrize("wall,sgs,wm,scheme,nwl", FORMS)
 def test_right_hand_sides(oracle_mod, wall, sgs, wm, scheme, nwl):
     c = _case(wall, sgs, wm, scheme, nwl)
-    state = cases.initial_condition(c)
+    state = _state(c)
     o = oracle_mod.Oracle(c)
     o.set_state(*state)
     if sgs:
@@ -49,7 +60,7 @@ def test_right_hand_sides(oracle_mod, wall, sgs, wm, scheme, nwl):
         s.close()
 
 
-@pytest.mark.parametrize("columns", [62, 64, 66, 130])
+@pytest.mark.parametrize("columns", [60, 64, 72, 128])
 @pytest.mark.parametrize("filt", [0, 1])
 def test_wall_model_columns(oracle_mod, columns, filt):
     c = _case(True, 2, 1, 0, nx=columns + 2, filt=filt)
