@@ -21,6 +21,7 @@
 #include "fft_smem.cuh"
 #include "kernels_diag.cuh"
 #include "kernels_fft2l.cuh"
+#include "kernels_plane.cuh"
 #include "kernels_poisson.cuh"
 #include "kernels_step.cuh"
 #include "kernels_hybrid.cuh"
@@ -122,6 +123,9 @@ struct dfdm_ctx {
     FFTPlan plan_x{}, plan_z{}, plan_y{};
     double *d_kxx = nullptr, *d_kzz = nullptr, *d_kyy = nullptr, *d_lo = nullptr, *d_di = nullptr, *d_up = nullptr;
     double *d_rpiv = nullptr;                   // 1/D(r) of every (kx,kz) tridiagonal system, layout (kz, r, kx)
+    double *d_rpivp = nullptr;                  // the same for k_plane, layout (kx, r, slot of kz)
+    // the spectrum is plane-major and k_plane replaces the z transforms and the y solve (plane_wins)
+    bool plane = false;
     double *d_dxc = nullptr, *d_dyc = nullptr, *d_dzc = nullptr;
     void *d_ub = nullptr;                       // streamwise base profile (storage type), zero in FP64
     bool ub_set = false;
@@ -405,7 +409,32 @@ template <int M> int row_lines(long long lines, int nsm, int per_sm = 3) {
     return lx;
 }
 template <typename T, int M> constexpr size_t row_smem(int lx) {
-    return (size_t)lx * RowLayout<M>::LD * sizeof(typename cplx_t<T>::type);
+    return (size_t)lx * RowLayout<M>::LDT * sizeof(typename cplx_t<T>::type);   // of either layout
+}
+// ---- k_plane: where it runs and how ----
+const size_t PLANE_SMEM_MAX = 232448;   // shared memory a block may use on sm_100
+// threads of a block: equal rounds of the first pass's items, at least the sweeps' 2 Nz
+int plane_block(const Dims &d) {
+    int n2 = 1;
+    with_fft2l(d.Nz, [&](auto n) { n2 = Split<decltype(n)::value>::N2; });
+    const int items = plane_rows(d.Ny) * n2, rounds = (items + PLANE_THREADS - 1) / PLANE_THREADS;
+    return (std::max(2 * d.Nz, (items + rounds - 1) / rounds) + 31) / 32 * 32;
+}
+bool two_level(int n) { return with_fft2l(n, [](auto) {}); }
+// Whether a stepping context runs k_plane: y walls, two-level x and z lengths, a half plane and its pivots within a block's
+// shared memory, and a shape where it measured faster.  FP32 / FP64 steps (graphed channel) against the three launches:
+// 128 x 96 x 128 cells 212 -> 182 / 354 -> 301 us, 16 x 190 x 96 177 -> 128 / 198 -> 158, 256 x 64 x 64 164 -> 151 / 255 ->
+// 246, 512 x 96 x 128 640 -> 575 / 1218 -> 1109.  Slower, and left to the three launches: small planes in many
+// (256 x 32 x 32 100 -> 103 / 129 -> 133: their launches fill the GPU and the pairs' exchange costs more), and Nz = 256
+// unless there are enough planes to fill the GPU once and no more (16 x 96 x 256 148 -> 150, 192 x 64 x 256 321 -> 339).
+// A plane larger than a pair of blocks holds was tried on clusters of two and four blocks sweeping in turn: 1070 -> 1280 us
+// at 256 x 192 x 256 (FP32).
+bool plane_wins(const Dims &d, int prec) {
+    if (d.yper || !two_level(d.Nx / 2) || !two_level(d.Nz)) return false;
+    const size_t sm = prec == DFDM_FP64 ? plane_smem<double>(d.Ny, d.Nz) : plane_smem<float>(d.Ny, d.Nz);
+    if (sm > PLANE_SMEM_MAX) return false;
+    if (d.Nxc > 49 && d.Ny * d.Nz < 48 * 48) return false;
+    return d.Nz < 256 || (d.Nxc >= 33 && 2 * d.Nxc <= 148);
 }
 // blocks of a column transform of `nl` columns each: the (j, kx) columns of the z transforms (families 3, 5) or the
 // (kz, kx) columns of the periodic-y solve (family 4)
@@ -435,9 +464,10 @@ template <typename T> struct Impl {
             c->thr_x2 = c->lx2 * Split<N>::N2;
             c->smem_x2 = row_smem<T, N>(c->lx2);
             const size_t cap = row_smem<T, N>(256 / Split<N>::N2);   // of every grid with this row length
-            setattr((const void *)k_fwd_x2<T, true, N>, cap);
-            setattr((const void *)k_fwd_x2<T, false, N>, cap);
-            setattr((const void *)k_inv_x2<T, N>, cap);
+            for (const void *fn : {(const void *)k_fwd_x2<T, true, N, false>, (const void *)k_fwd_x2<T, true, N, true>,
+                                   (const void *)k_fwd_x2<T, false, N, false>, (const void *)k_fwd_x2<T, false, N, true>,
+                                   (const void *)k_inv_x2<T, N, false>, (const void *)k_inv_x2<T, N, true>})
+                setattr(fn, cap);
         });
         c->z2 = with_fft2l(d.Nz, [&](auto n) {
             constexpr int N = decltype(n)::value;
@@ -446,6 +476,11 @@ template <typename T> struct Impl {
             setattr((const void *)k_col2<T, 0, NL, N>, c->smem_z2);
             setattr((const void *)k_col2<T, 1, NL, N>, c->smem_z2);
         });
+        if (c->plane)
+            with_fft2l(d.Nz, [&](auto n) {
+                constexpr int N = decltype(n)::value;
+                setattr((const void *)k_plane<T, N>, PLANE_SMEM_MAX);
+            });
         c->y2 = d.yper && with_fft2l(d.Ny, [&](auto n) {
             constexpr int N = decltype(n)::value;
             c->smem_y2 = (size_t)2 * N * NL * sizeof(C);
@@ -464,12 +499,10 @@ template <typename T> struct Impl {
             const int nb = (int)((lines + c->lx2 - 1) / c->lx2);
             with_fft2l(d.Nx / 2, [&](auto n) {
                 constexpr int N = decltype(n)::value;
-                if (from_div)
-                    k_fwd_x2<T, true, N><<<nb, c->thr_x2, c->smem_x2, st>>>(poisson_args<T>(c), c->lx2, f(c->us), f(c->vs), f(c->wsf),
-                                                                       nullptr, (C *)c->spec, (const C *)c->tw_x, (const C *)c->twr_x);
-                else
-                    k_fwd_x2<T, false, N><<<nb, c->thr_x2, c->smem_x2, st>>>(poisson_args<T>(c), c->lx2, nullptr, nullptr, nullptr,
-                                                                        src, (C *)c->spec, (const C *)c->tw_x, (const C *)c->twr_x);
+                auto fn = from_div ? (c->plane ? k_fwd_x2<T, true, N, true> : k_fwd_x2<T, true, N, false>)
+                                   : (c->plane ? k_fwd_x2<T, false, N, true> : k_fwd_x2<T, false, N, false>);
+                fn<<<nb, c->thr_x2, c->smem_x2, st>>>(poisson_args<T>(c), c->lx2, f(c->us), f(c->vs), f(c->wsf), src,
+                                                      (C *)c->spec, (const C *)c->tw_x, (const C *)c->twr_x);
             });
         } else {
             const int nb = (int)((lines + c->lx - 1) / c->lx);
@@ -959,7 +992,8 @@ template <typename T> struct Impl {
         }
         case 2:   // div + forward x
             return fwd_x(c, true, nullptr);
-        case 3: case 5: {   // z transforms
+        case 3: case 5: {   // z transforms (with k_plane: part of family 4)
+            if (c->plane) return DFDM_OK;
             if (c->z2) {
                 const int g = col_blocks(d, which, NL);
                 with_fft2l(d.Nz, [&](auto n) {
@@ -982,7 +1016,13 @@ template <typename T> struct Impl {
             return DFDM_OK;
         }
         case 4: {   // y solve
-            if (d.yper && c->y2) {
+            if (c->plane) {
+                with_fft2l(d.Nz, [&](auto n) {
+                    constexpr int L = decltype(n)::value;
+                    k_plane<T, L><<<2 * d.Nxc, plane_block(d), plane_smem<T>(d.Ny, d.Nz), st>>>(
+                        d, (C *)c->spec, (const C *)c->tw_z, c->d_rpivp, c->d_lo, c->d_up);
+                });
+            } else if (d.yper && c->y2) {
                 const int g = col_blocks(d, which, NL);
                 with_fft2l(d.Ny, [&](auto n) {
                     constexpr int N = decltype(n)::value;
@@ -1009,8 +1049,9 @@ template <typename T> struct Impl {
                 int nb = (int)((lines + c->lx2 - 1) / c->lx2);
                 with_fft2l(d.Nx / 2, [&](auto n) {
                     constexpr int N = decltype(n)::value;
-                    k_inv_x2<T, N><<<nb, c->thr_x2, c->smem_x2, st>>>(poisson_args<T>(c), c->lx2, (const C *)c->spec, f(c->phi),
-                                                                  (const C *)c->tw_x, (const C *)c->twr_x);
+                    auto fn = c->plane ? k_inv_x2<T, N, true> : k_inv_x2<T, N, false>;
+                    fn<<<nb, c->thr_x2, c->smem_x2, st>>>(poisson_args<T>(c), c->lx2, (const C *)c->spec, f(c->phi),
+                                                          (const C *)c->tw_x, (const C *)c->twr_x);
                 });
             } else {
                 int nb = (int)((lines + c->lx - 1) / c->lx);
@@ -1278,6 +1319,21 @@ bool fuse_eligible(const dfdm_params *p) {
     return (p->flat_wall_model_flag == 0 || p->wm_filter_mode != 0) && p->advection_scheme != 2;
 }
 
+// the sizes of a stepping grid that the choice of kernels looks at
+Dims grid_dims(const dfdm_grid *g) {
+    Dims d{};
+    d.yper = g->y_bc_type == 0;
+    d.Nx = g->nx - 2; d.Nz = g->nz - 2;
+    d.Ny = d.yper ? g->ny - 2 : g->ny - 1;
+    d.Nxc = d.Nx / 2 + 1;
+    return d;
+}
+
+// the model a serving group's members may have (group_create checks the rest)
+bool group_takes(const dfdm_params *p) {
+    return p->precision == DFDM_FP32_MIXED && p->sgs_model == 0 && p->flat_wall_model_flag == 0 && p->advection_scheme != 2;
+}
+
 // Bytes of the buffers dfdm_create carves from the context's arena (every sub-allocation 256-byte aligned).
 size_t arena_bytes(const dfdm_grid *g, const dfdm_params *p) {
     size_t ts = p->precision == DFDM_FP64 ? 8 : 4;
@@ -1303,7 +1359,8 @@ size_t arena_bytes(const dfdm_grid *g, const dfdm_params *p) {
                              (p->advection_scheme == 2 ? 3 /*hybrid-scheme terms*/ : 0) +
                              (fuse_eligible(p) ? 3 /*second u* set*/ : 0));
     n += spec * 2 * ts;
-    if (g->y_bc_type != 0) n += (Nx / 2 + 1) * Ny * Nz * 8;   // pivot table of the y solves
+    // pivot table of the y solves; a second one where k_plane runs and a group may too
+    if (g->y_bc_type != 0) n += (Nx / 2 + 1) * Ny * Nz * 8 * (group_takes(p) && plane_wins(grid_dims(g), p->precision) ? 2 : 1);
     n += 9 * Nx * Nz * 2 * 8;   // wall planes (and the eddy viscosity's wall factors)
     n += 1 << 20;               // metrics, twiddles, reductions, alignment
     return n;
@@ -1596,6 +1653,7 @@ int dfdm_create(const dfdm_grid *g, const dfdm_params *prm, dfdm_ctx **out) {
     d.yper = c->yper;
     d.plane = (long long)d.Nx * d.Ny;
     d.cells = d.plane * d.Nz;
+    c->plane = plane_wins(d, c->prec);
     // automatic defaults (src/input_output.f90:938-940, :967-970)
     c->nwl = prm->adv_wall_layers;
     if (c->nwl < 0) { c->nwl = 0; if (prm->flat_wall_model_flag > 0 && prm->advection_scheme != 1) c->nwl = 8; }
@@ -1725,24 +1783,21 @@ int dfdm_create(const dfdm_grid *g, const dfdm_params *prm, dfdm_ctx **out) {
     if ((rc = upload_as<double>(c, &tmp, up))) return bail(rc);
     c->d_up = (double *)tmp;
     if (!c->yper) {
-        // pivots of the no-interchange zgtsv elimination of every (kx,kz) system (src/projection.f90:284-295)
-        std::vector<double> rpiv((size_t)d.Nxc * d.Ny * d.Nz);
-        for (int kz = 0; kz < d.Nz; ++kz)
-            for (int kx = 0; kx < d.Nxc; ++kx) {
-                double lam = kxx[kx] + kzz[kz];
-                double D = di[0] + lam;
-                if (kx == 0 && kz == 0) D = 3.0 / 2.0 * D;
-                size_t b = (size_t)kz * d.Ny * d.Nxc + kx;
-                rpiv[b] = 1.0 / D;
-                for (int r = 1; r < d.Ny; ++r) {
-                    double m = lo[r] / D;
-                    D = (di[r] + lam) - m * up[r - 1];
-                    if (D == 0.0) return bail(fail(DFDM_ERR_INVALID, "singular pressure operator"));
-                    rpiv[b + (size_t)r * d.Nxc] = 1.0 / D;
-                }
-            }
-        if ((rc = upload_as<double>(c, &tmp, rpiv))) return bail(rc);
-        c->d_rpiv = (double *)tmp;
+        // pivots of the no-interchange zgtsv elimination of every (kx,kz) system (src/projection.f90:284-295): for k_plane's
+        // solve, for the others, or for both where a serving group's launches read a k_plane context's table
+        const size_t n = (size_t)d.Nxc * d.Ny * d.Nz;
+        if ((!c->plane || group_takes(prm)) && (rc = dalloc(c, (void **)&c->d_rpiv, n * sizeof(double)))) return bail(rc);
+        if (c->plane && (rc = dalloc(c, (void **)&c->d_rpivp, n * sizeof(double)))) return bail(rc);
+        if ((rc = dalloc(c, &tmp, sizeof(int)))) return bail(rc);   // zeroed
+        int n1 = 1, n2 = d.Nz, bad = 0;
+        with_fft2l(d.Nz, [&](auto L) { n1 = Split<decltype(L)::value>::N1; n2 = Split<decltype(L)::value>::N2; });
+        k_pivots<<<dim3((d.Nxc + 127) / 128, d.Nz), 128, 0, c->stream>>>(d, n1, n2, c->d_kxx, c->d_kzz, c->d_lo, c->d_di, c->d_up,
+                                                                         c->d_rpiv, c->d_rpivp, (int *)tmp);
+        if (cudaGetLastError() != cudaSuccess ||
+            cudaMemcpyAsync(&bad, tmp, sizeof(int), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
+            cudaStreamSynchronize(c->stream) != cudaSuccess)
+            return bail(fail(DFDM_ERR_CUDA, "the pivot tables of the y solve could not be made"));
+        if (bad) return bail(fail(DFDM_ERR_INVALID, "singular pressure operator"));
     }
 
     // ---- FFT plans and twiddles ----
@@ -2959,7 +3014,8 @@ int dfdm_kernel_bytes(dfdm_ctx *c, int which, double *bytes) {
     case 1: b = 12.0 * cell + (c->les ? cell : 0.0) + (c->fused ? cell : 0.0); break;   // stage 1: 3 in, 9 out; stages 2/3:
                                                                   // 9 in, 3 out (fused corrections: + phi)
     case 2: b = 3.0 * cell + spec; break;                         // read u*, write spectrum
-    case 3: case 4: case 5: b = 2.0 * spec; break;                // read + write spectrum
+    case 3: case 5: b = c->plane ? 0.0 : 2.0 * spec; break;       // read + write spectrum (k_plane: family 4 alone)
+    case 4: b = 2.0 * spec; break;
     case 6: b = spec + cell; break;                               // read spectrum, write phi
     case 7: b = 7.0 * cell; break;                                // read phi, u*; write u (+P at stage 3)
     case 9: b = c->prm.flow_forcing_mode == 1 ? 3.0 * cell : 0.0; break;   // bulk sum reads U; the shift reads + writes U

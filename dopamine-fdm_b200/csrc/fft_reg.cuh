@@ -115,11 +115,12 @@ template <typename F> inline bool with_fft2l(int n, F &&f) {
 
 // Shared memory of the row transforms (x lines), in complex elements: line ll at ll * LD, holding either the line in
 // natural order or the step-1 outputs, element k1*N2 + n2 at k1*(N2+1) + n2.  LD is 8 mod 16, so that two lines in one
-// half-warp use disjoint banks.
+// half-warp use disjoint banks; LDT, of the kernels that also access one element of many lines at once (the plane-major
+// spectrum), is 9 mod 16: odd, so that those accesses spread over all banks.
 template <int N> struct RowLayout {
     static constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
     static constexpr int pad8(int x) { return x + ((8 - (x % 16) + 16) % 16); }
-    static constexpr int LD = pad8(N1 * (N2 + 1));
+    static constexpr int LD = pad8(N1 * (N2 + 1)), LDT = LD + 1;
 };
 
 // Step 1 of a row transform for one (line, n2) item: v holds x[n1*N2 + n2], n1 = 0..N1-1, on entry; the twiddled

@@ -27,7 +27,7 @@ template <int Q> struct RowGroup {
 // by the latency of its phases more than by bandwidth: pairs of cells with per-pair indexing and two buffers (fewer lines
 // per block) took 62 us at 256 x 192 x 256 cells in FP32 and 145 us in FP64, this form 46 and 105 us (207 MB of traffic in
 // FP32: 0.69 of the measured copy bandwidth).
-template <typename T, bool FROM_DIV, int M, class BC>
+template <typename T, bool FROM_DIV, int M, bool TR = false, class BC>
 __device__ __forceinline__ void k_fwd_x2_body(const BC &bc, const PoissonArgs<T> &a, int lx, const T *__restrict__ U, const T *__restrict__ V,
                                                 const T *__restrict__ W_, const T *__restrict__ src,
                                                 typename cplx_t<T>::type *__restrict__ spec,
@@ -36,7 +36,7 @@ __device__ __forceinline__ void k_fwd_x2_body(const BC &bc, const PoissonArgs<T>
     typedef typename cplx_t<T>::type C;
     typedef Arith<T> A;
     constexpr int N1 = Split<M>::N1, N2 = Split<M>::N2, Nx = 2 * M;
-    constexpr int LD = RowLayout<M>::LD;
+    constexpr int LD = TR ? RowLayout<M>::LDT : RowLayout<M>::LD;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *buf = (C *)smem_raw;
     const Dims &d = a.d;
@@ -49,6 +49,10 @@ __device__ __forceinline__ void k_fwd_x2_body(const BC &bc, const PoissonArgs<T>
     // line's indices, metrics and row pointers are formed once per lane and line
     constexpr int W = 16 / (int)sizeof(T), Q = Nx / W, G = RowGroup<Q>::value, NQ = Q / G, UNR = NQ % 2 == 0 ? 2 : 1;
     struct alignas(16) Vec { T x[W]; };
+    auto put = [](C *p, const Vec &z) {   // lines of the TR form start on 8-byte boundaries only (FP32)
+        if constexpr (TR && W == 4) { p[0] = mkc<T>(z.x[0], z.x[1]); p[1] = mkc<T>(z.x[2], z.x[3]); }
+        else *reinterpret_cast<Vec *>(p) = z;
+    };
     const int lane = threadIdx.x % G;
     for (int ll = threadIdx.x / G; ll < nl; ll += blockDim.x / G) {
         const int line = line0 + ll;
@@ -82,14 +86,13 @@ __device__ __forceinline__ void k_fwd_x2_body(const BC &bc, const PoissonArgs<T>
                         z.x[x] = (u[q].x[x] - (x == 0 ? um[q] : u[q].x[x - 1])) * a.inv_dx + (v[q].x[x] - vb) * riy +
                                  (w[q].x[x] - wm[q].x[x]) * riz;
                     }
-                    *reinterpret_cast<Vec *>(zl + (c0 + q) * G * (W / 2)) = z;
+                    put(zl + (c0 + q) * G * (W / 2), z);
                 }
             }
         } else {
             const T *row = src + (size_t)line * Nx + lane * W;
 #pragma unroll
-            for (int c = 0; c < NQ; ++c)
-                *reinterpret_cast<Vec *>(zl + c * G * (W / 2)) = *reinterpret_cast<const Vec *>(row + c * G * W);
+            for (int c = 0; c < NQ; ++c) put(zl + c * G * (W / 2), *reinterpret_cast<const Vec *>(row + c * G * W));
         }
     }
     __syncthreads();
@@ -130,9 +133,13 @@ __device__ __forceinline__ void k_fwd_x2_body(const BC &bc, const PoissonArgs<T>
     }
     __syncthreads();
     const int Nxc = d.Nxc;
-    // modes k and M-k together: with E, O as k_fwd_x forms them, X_k = E + W^k O and X_{M-k} = conj(E - W^k O)
-    for (int e = threadIdx.x; e < nl * (M / 2 + 1); e += blockDim.x) {
-        const int ll = e / (M / 2 + 1), k = e - ll * (M / 2 + 1);
+    // modes k and M-k together: with E, O as k_fwd_x forms them, X_k = E + W^k O and X_{M-k} = conj(E - W^k O).  Consecutive
+    // threads take consecutive modes of a line, or (TR) one mode of consecutive lines: the spectrum's contiguous index
+    constexpr int H = M / 2 + 1;
+    const size_t nlines = (size_t)Ny * Nz;
+    for (int e = threadIdx.x; e < (TR ? lx : nl) * H; e += blockDim.x) {
+        const int ll = TR ? e & (lx - 1) : e / H, k = TR ? e / lx : e - ll * H;   // lx is a power of two
+        if (TR && ll >= nl) continue;
         const C *res = buf + ll * LD;
         const C Zk = res[k], Zm = res[k == 0 ? 0 : M - k];
         const T Er = T(0.5) * (Zk.x + Zm.x), Ei = T(0.5) * (Zk.y - Zm.y);
@@ -140,44 +147,47 @@ __device__ __forceinline__ void k_fwd_x2_body(const BC &bc, const PoissonArgs<T>
         const T Or = Di, Oi = -Dr;
         const C w = __ldg(twr + k);
         const T Pr = w.x * Or - w.y * Oi, Pi = w.x * Oi + w.y * Or;
-        C *row = spec + (size_t)(line0 + ll) * Nxc;
-        row[k] = mkc<T>(Er + Pr, Ei + Pi);
-        if (2 * k != M) row[M - k] = mkc<T>(Er - Pr, Pi - Ei);
+        C *row = TR ? spec + line0 + ll : spec + (size_t)(line0 + ll) * Nxc;
+        const size_t ks = TR ? nlines : 1;
+        row[k * ks] = mkc<T>(Er + Pr, Ei + Pi);
+        if (2 * k != M) row[(M - k) * ks] = mkc<T>(Er - Pr, Pi - Ei);
     }
 }
-template <typename T, bool FROM_DIV, int M>
+template <typename T, bool FROM_DIV, int M, bool TR>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_fwd_x2(PoissonArgs<T> a, int lx, const T *__restrict__ U, const T *__restrict__ V,
                                                 const T *__restrict__ W, const T *__restrict__ src,
                                                 typename cplx_t<T>::type *__restrict__ spec,
                                                 const typename cplx_t<T>::type *__restrict__ tw,
                                                 const typename cplx_t<T>::type *__restrict__ twr) {
     pdl_enter();
-    k_fwd_x2_body<T, FROM_DIV, M>(HwBlock(), a, lx, U, V, W, src, spec, tw, twr);
+    k_fwd_x2_body<T, FROM_DIV, M, TR>(HwBlock(), a, lx, U, V, W, src, spec, tw, twr);
 }
 
 // ---- inverse complex-to-real x transform, writes phi = x / (nxp*nzp) -----------------------------------------
-template <typename T, int M, class BC>
+template <typename T, int M, bool TR = false, class BC>
 __device__ __forceinline__ void k_inv_x2_body(const BC &bc, const PoissonArgs<T> &a, int lx, const typename cplx_t<T>::type *__restrict__ spec,
                                                 T *__restrict__ phi, const typename cplx_t<T>::type *__restrict__ tw,
                                                 const typename cplx_t<T>::type *__restrict__ twr) {
     typedef typename cplx_t<T>::type C;
     typedef typename Vec2<T>::type T2;
     constexpr int N1 = Split<M>::N1, N2 = Split<M>::N2, Nx = 2 * M;
-    constexpr int LD = RowLayout<M>::LD;
+    constexpr int LD = TR ? RowLayout<M>::LDT : RowLayout<M>::LD;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *bt = (C *)smem_raw;
     const Dims &d = a.d;
     const int Nxc = d.Nxc;
     const int line0 = bc.idx().x * lx;
     const int nl = min(lx, d.Ny * d.Nz - line0);
-    for (int b = threadIdx.x; b < nl * N2; b += blockDim.x) {
-        const int ll = b / N2, n2 = b - ll * N2;
-        const C *row = spec + (size_t)(line0 + ll) * Nxc;
+    const size_t ks = TR ? (size_t)d.Ny * d.Nz : 1;   // between modes; TR: consecutive threads on consecutive lines
+    for (int b = threadIdx.x; b < (TR ? lx : nl) * N2; b += blockDim.x) {
+        const int ll = TR ? b & (lx - 1) : b / N2, n2 = TR ? b / lx : b - ll * N2;   // lx is a power of two
+        if (TR && ll >= nl) continue;
+        const C *row = TR ? spec + line0 + ll : spec + (size_t)(line0 + ll) * Nxc;
         C v[N1];
 #pragma unroll
         for (int n1 = 0; n1 < N1; ++n1) {
             const int kx = n1 * N2 + n2;
-            C X = row[kx], Xm = row[M - kx];
+            C X = row[kx * ks], Xm = row[(M - kx) * ks];
             if (kx == 0) { X.y = T(0); Xm.y = T(0); }
             T E2r = X.x + Xm.x, E2i = X.y - Xm.y;
             T D2r = X.x - Xm.x, D2i = X.y + Xm.y;
@@ -211,12 +221,12 @@ __device__ __forceinline__ void k_inv_x2_body(const BC &bc, const PoissonArgs<T>
         }
     }
 }
-template <typename T, int M>
+template <typename T, int M, bool TR>
 __global__ void __launch_bounds__(256) k_inv_x2(PoissonArgs<T> a, int lx, const typename cplx_t<T>::type *__restrict__ spec,
                                                 T *__restrict__ phi, const typename cplx_t<T>::type *__restrict__ tw,
                                                 const typename cplx_t<T>::type *__restrict__ twr) {
     pdl_enter();
-    k_inv_x2_body<T, M>(HwBlock(), a, lx, spec, phi, tw, twr);
+    k_inv_x2_body<T, M, TR>(HwBlock(), a, lx, spec, phi, tw, twr);
 }
 
 // ---- z transforms (MODE 0 forward, 1 inverse) and the periodic-y solve (MODE 2) on tiles of NL columns ----

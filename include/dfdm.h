@@ -292,7 +292,8 @@ int dfdm_pad_field(dfdm_ctx *ctx, int field, int extra_planes, double *out);
 /* ---- profiling hooks: launch one kernel family of one RK stage on the context's stream, no sync ----
  * which: 0 SGS, 1 stage (RHS + RK update), 2 div + forward x-FFT, 3 forward z-FFT, 4 y solve,
  *        5 inverse z-FFT, 6 inverse x-FFT, 7 velocity correction, 8 wall model, 9 constant-flux bulk sum + shift,
- *        10 CFL maxima, 11 the dissipative terms of advection_scheme = 2 */
+ *        10 CFL maxima, 11 the dissipative terms of advection_scheme = 2.  On wall-bounded grids whose z transforms and y
+ *        solve run as one launch (small and middle sizes) that launch is family 4; 3 and 5 launch nothing there. */
 int dfdm_launch_kernel_async(dfdm_ctx *ctx, int which, int rk_stage);
 /* Fused corrections (on by default where they apply: the wall model only with its temporal filter, no hybrid
  * advection scheme; LES only with the eddy viscosity computed in the stage tiles, dfdm_set_sgs_in_tile).  The projections of RK stages 1
