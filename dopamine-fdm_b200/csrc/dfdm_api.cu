@@ -116,6 +116,7 @@ struct dfdm_ctx {
     bool fuse_ok = false, fused = false;
     void *nut = nullptr, *p = nullptr, *phi = nullptr, *spec = nullptr, *rhs3 = nullptr;
     void *my_t = nullptr, *mz_t = nullptr;      // 6 metric arrays each, storage type
+    double *zmd = nullptr, *ymd = nullptr;      // FP64: the same values per z plane and y row (StepArgs::zmd, ymd)
     void *zm8 = nullptr;                        // FP32: the z metrics of each plane in load_pairs order (StepArgs::zm8)
     double *d_wfac = nullptr;                   // LES + wall model: wall factors of the eddy viscosity (k_wall_sgs)
     double *my_d = nullptr, *mz_d = nullptr;    // same in double
@@ -344,6 +345,8 @@ template <typename T> StepArgs<T> step_args(dfdm_ctx *c) {
     a.adv = (const T *)c->adv;
     a.phi = (const T *)c->phi;
     a.zm8 = (const float *)c->zm8;
+    a.zmd = c->zmd;
+    a.ymd = c->ymd;
     a.wfac = c->d_wfac;
     return a;
 }
@@ -1362,6 +1365,7 @@ size_t arena_bytes(const dfdm_grid *g, const dfdm_params *p) {
     // pivot table of the y solves; a second one where k_plane runs and a group may too
     if (g->y_bc_type != 0) n += (Nx / 2 + 1) * Ny * Nz * 8 * (group_takes(p) && plane_wins(grid_dims(g), p->precision) ? 2 : 1);
     n += 9 * Nx * Nz * 2 * 8;   // wall planes (and the eddy viscosity's wall factors)
+    n += 64 * (Ny + Nz);        // the axes' metrics in the stage kernels' order (zm8; zmd, ymd)
     n += 1 << 20;               // metrics, twiddles, reductions, alignment
     return n;
 }
@@ -1703,19 +1707,27 @@ int dfdm_create(const dfdm_grid *g, const dfdm_params *prm, dfdm_ctx **out) {
     c->my_d = (double *)tmp;
     if ((rc = upload_as<double>(c, &tmp, mz))) return bail(rc);
     c->mz_d = (double *)tmp;
-    if (c->prec == DFDM_FP64) { c->my_t = c->my_d; c->mz_t = c->mz_d; }
-    else {
+    // the eight metrics around index p of an axis with n cells: w0, w1 at p-1 and p, idc at p and p+1, idf at p-1 and p
+    auto around = [](const std::vector<double> &m, int n, int p, int t) {
+        const int src[8][2] = {{2, p - 1}, {3, p - 1}, {2, p}, {3, p}, {4, p}, {4, p + 1}, {5, p - 1}, {5, p}};
+        return m[(size_t)src[t][0] * (n + 3) + 1 + src[t][1]];
+    };
+    if (c->prec == DFDM_FP64) {
+        c->my_t = c->my_d;
+        c->mz_t = c->mz_d;
+        std::vector<double> zd((size_t)d.Nz * 8), yd((size_t)d.Ny * 8);
+        for (int k = 0; k < d.Nz; ++k)
+            for (int t = 0; t < 8; ++t) zd[(size_t)k * 8 + t] = around(mz, d.Nz, k, t);
+        for (int j = 0; j < d.Ny; ++j)
+            for (int t = 0; t < 8; ++t) yd[(size_t)j * 8 + t] = around(my, d.Ny, j, t);
+        if ((rc = upload_as<double>(c, (void **)&c->zmd, zd)) || (rc = upload_as<double>(c, (void **)&c->ymd, yd))) return bail(rc);
+    } else {
         if ((rc = upload_as<float>(c, &c->my_t, my))) return bail(rc);
         if ((rc = upload_as<float>(c, &c->mz_t, mz))) return bail(rc);
-        // per plane k: w0(k-1), w1(k-1), w0(k), w1(k), idc(k), idc(k+1), idf(k-1), idf(k) of metric_view's layout
-        // (AxisLocal<F2>::load_pairs), each twice, the same FP32 values as mz_t
-        const int L = d.Nz + 3;
+        // per plane, each twice, the same FP32 values as mz_t (AxisLocal<F2>::load_pairs)
         std::vector<double> z8((size_t)d.Nz * ZPAIRS);
-        for (int k = 0; k < d.Nz; ++k) {
-            const int src[8][2] = {{2, k - 1}, {3, k - 1}, {2, k}, {3, k}, {4, k}, {4, k + 1}, {5, k - 1}, {5, k}};
-            for (int t = 0; t < 8; ++t)
-                z8[(size_t)k * ZPAIRS + 2 * t] = z8[(size_t)k * ZPAIRS + 2 * t + 1] = mz[(size_t)src[t][0] * L + 1 + src[t][1]];
-        }
+        for (int k = 0; k < d.Nz; ++k)
+            for (int t = 0; t < 8; ++t) z8[(size_t)k * ZPAIRS + 2 * t] = z8[(size_t)k * ZPAIRS + 2 * t + 1] = around(mz, d.Nz, k, t);
         if ((rc = upload_as<float>(c, &c->zm8, z8))) return bail(rc);
     }
     std::vector<double> dxc(d.Nx), dyc(d.Ny), dzc(d.Nz);

@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(les::NT, 2) k_les(StepArgs<T> a, const T *__re
 #pragma unroll
     for (int dj = -1; dj <= 1; ++dj) ubr[dj + 1] = ub_row(min(j, Ny - 1) + dj);
     AxisLocal<T> Y;
-    Y.load(a.my, min(j, Ny - 1));
+    if constexpr (sizeof(T) == 8) Y.v = a.ymd + 8 * min(j, Ny - 1); else Y.load(a.my, min(j, Ny - 1));
     RowProfile<T> R;
     R.load(ubr, Y, row_wd<T, WM>(a, j));
 
@@ -232,7 +232,9 @@ __global__ void __launch_bounds__(les::NT, 2) k_les(StepArgs<T> a, const T *__re
             q.v[0] = vel(1, vslot(k - 1)); q.v[1] = vel(1, vslot(k)); q.v[2] = vel(1, vslot(k + 1));
             q.w[0] = vel(2, vslot(k - 1)); q.w[1] = vel(2, vslot(k)); q.w[2] = vel(2, vslot(k + 1));
             q.n[0] = smn + nslot(k - 1) * PS; q.n[1] = smn + nslot(k) * PS; q.n[2] = smn + nslot(k + 1) * PS;
-            stage_cell<T, true, WM, false>(a, q, Y, R, tau_x, tau_z, sc, i, j, k, uo, vo, wo, f1u, f1v, f1w, us, vs, wsf,
+            const T *zm = nullptr;
+            if constexpr (sizeof(T) == 8) zm = a.zmd + 8 * k;
+            stage_cell<T, true, WM, false>(a, q, Y, R, zm, tau_x, tau_z, sc, i, j, k, uo, vo, wo, f1u, f1v, f1w, us, vs, wsf,
                                            nullptr);
             if (nut_out) nut_out[k * plane + j * Nx + i] = q.N(0, 0, 0);   // stage 3: the step's last nu_t, kept
         }

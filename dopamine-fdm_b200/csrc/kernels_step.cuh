@@ -74,6 +74,8 @@ template <typename T> struct StepArgs {
     // FP32: the eight z metrics of every plane in AxisLocal<F2>::load_pairs order, each twice: ZPAIRS consecutive values
     // per plane (copied to shared memory with the plane); null in FP64
     const float *zm8;
+    // FP64: the same eight values per z plane and per y row, once each; null in FP32
+    const double *zmd, *ymd;
     // LES with the wall model: the first-cell gradient factor of every wall cell, (iw*Nz + k)*Nx + i, written by
     // k_wall_sgs from the velocity the eddy viscosity is computed from (NaN where the override does not apply);
     // null: nut_at solves for it in place
@@ -227,7 +229,7 @@ __global__ void __launch_bounds__(WALL_THREADS) k_wall_model(StepArgs<T> a, Wall
 // ---------------------------------------------------------------------------------------------------------------
 // Metric values around one index p of an axis: weights of faces p-1 and p, widths and spacings at p-1, p, p+1.
 // FP32 reads them once per thread (y) or once per plane (z) and keeps them in registers; FP64 reads them where
-// they are used (its registers are taken by the double-precision stencil).
+// they are used (its registers are taken by the double-precision stencil), k_tiled from shared memory.
 constexpr int ZPAIRS = 16;   // floats of one plane's z metrics in load_pairs order
 template <typename T> struct AxisLocal;
 template <> struct AxisLocal<float> {
@@ -268,17 +270,15 @@ template <> struct AxisLocal<F2> {   // packed pairs: the same metrics broadcast
     __device__ __forceinline__ F2 invfm() const { return idfm_; }
 };
 template <> struct AxisLocal<double> {
-    const Metric1D<double> *m;   // the kernel argument's metric (stays in the parameter bank once inlined)
-    int p;
-    __device__ __forceinline__ void load(const Metric1D<double> &m_, int p_) { m = &m_; p = p_; }
-    __device__ __forceinline__ double w0m() const { return m->w0[p - 1]; }
-    __device__ __forceinline__ double w1m() const { return m->w1[p - 1]; }
-    __device__ __forceinline__ double w0() const { return m->w0[p]; }
-    __device__ __forceinline__ double w1() const { return m->w1[p]; }
-    __device__ __forceinline__ double invc() const { return m->idc[p]; }
-    __device__ __forceinline__ double invcp() const { return m->idc[p + 1]; }
-    __device__ __forceinline__ double invf() const { return m->idf[p]; }
-    __device__ __forceinline__ double invfm() const { return m->idf[p - 1]; }
+    const double *v;   // the eight values of load_pairs' order, once each (shared memory in k_tiled, else StepArgs::zmd, ymd)
+    __device__ __forceinline__ double w0m() const { return v[0]; }
+    __device__ __forceinline__ double w1m() const { return v[1]; }
+    __device__ __forceinline__ double w0() const { return v[2]; }
+    __device__ __forceinline__ double w1() const { return v[3]; }
+    __device__ __forceinline__ double invc() const { return v[4]; }
+    __device__ __forceinline__ double invcp() const { return v[5]; }
+    __device__ __forceinline__ double invfm() const { return v[6]; }
+    __device__ __forceinline__ double invf() const { return v[7]; }
 };
 
 // The gradient factor of the eddy viscosity's wall override for every wall cell (wall_gradient_factor), from the
@@ -572,8 +572,8 @@ template <int PX> struct TileQ2 {
 // update (or, with rhs_only, the right-hand sides themselves).  Shared by the one-cell stage kernels.
 template <typename T, bool LES, bool WM, bool HYB, typename Q>
 __device__ __forceinline__ void stage_cell(const StepArgs<T> &a, const Q &q, const AxisLocal<T> &Y,
-                                           const RowProfile<T> &R, const double *__restrict__ tau_x, const double *__restrict__ tau_z,
-                                           const StageCoef &sc, int i, int j, int k, T *__restrict__ uo,
+                                           const RowProfile<T> &R, const T *zm, const double *__restrict__ tau_x,
+                                           const double *__restrict__ tau_z, const StageCoef &sc, int i, int j, int k, T *__restrict__ uo,
                                            T *__restrict__ vo, T *__restrict__ wo, T *__restrict__ f1u,
                                            T *__restrict__ f1v, T *__restrict__ f1w, T *__restrict__ us,
                                            T *__restrict__ vs, T *__restrict__ wsf, T *__restrict__ rhs_only) {
@@ -588,7 +588,7 @@ __device__ __forceinline__ void stage_cell(const StepArgs<T> &a, const Q &q, con
         if (vrow) fv = f1v[p];
     }
     AxisLocal<T> Z;
-    Z.load(a.mz, k);
+    if constexpr (sizeof(T) == 8) Z.v = zm; else Z.load(a.mz, k);
     T ru, rv, rw;
     rhs_at<T, LES, WM>(a, q, Y, R, Z, tau_x, tau_z, i, j, k, vrow, ru, rv, rw);
     if constexpr (HYB) {
@@ -646,11 +646,20 @@ __device__ __forceinline__ void k_tiled_body(const BC &bc, const StepArgs<T> &a,
     __shared__ __align__(16) T sm[NF][4][PS];
     constexpr int PXP = PX + 1, PSP = PXP * (PY + 1), PERP = (PSP + NT - 1) / NT;   // phi tile: one more column, row
     __shared__ __align__(16) T smp[CORR ? 5 : 1][CORR ? PSP : 1];
+    // FP64: the metrics of the tile's rows and, in a ring, of planes k .. k+2.  A thread reads each value several times per
+    // cell, and read from the global tables they were the kernel's longest stall: a step took 2296 us at 256 x 192 x 256
+    // (2166 from shared memory) and 301 us at 128 x 94 x 128 (285)
+    constexpr bool MS = sizeof(T) == 8 && KIND != 1;
+    __shared__ double ymr[MS ? TY * 8 : 1], zmr[MS ? 4 : 1][8];
     const Dims &d = a.d;
     const int Nx = d.Nx, Ny = d.Ny, Nz = d.Nz;
     const int i0 = bc.idx().x * TX, j0 = bc.idx().y * TY;
     const int k0 = bc.idx().z * kc, kend = min(k0 + kc, Nz);
     const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
+    auto issue_z = [&](int k) {   // the z metrics of plane k (k0 <= k < kend) into zmr[(k - k0) & 3]
+        if constexpr (MS)
+            if (threadIdx.x < 8 && k < kend) cp_async<8>(&zmr[(k - k0) & 3][threadIdx.x], a.zmd + 8 * k + threadIdx.x);
+    };
     const int i = i0 + tx, j = j0 + ty;
     const bool active = i < Nx && j < Ny;
     const int plane = Nx * Ny;
@@ -762,13 +771,19 @@ __device__ __forceinline__ void k_tiled_body(const BC &bc, const StepArgs<T> &a,
     }
 
     AxisLocal<T> Y;   // this thread's y metrics (FP32: read here once for every plane)
-    Y.load(a.my, min(j, Ny - 1));
+    if constexpr (sizeof(T) == 8 && KIND != 1) {
+        for (int e = threadIdx.x; e < TY * 8; e += NT) ymr[e] = a.ymd[min(j0 + e / 8, Ny - 1) * 8 + e % 8];
+        Y.v = reinterpret_cast<const double *>(ymr) + 8 * ty;
+    } else if constexpr (sizeof(T) == 4) {
+        Y.load(a.my, min(j, Ny - 1));
+    }
     RowProfile<T> R;
     R.load(ubr, Y, row_wd<T, WM>(a, j));
 
     // planes k0-1, k0, k0+1 into slots 0, 1, 2; plane k lives in slot (k - k0 + 1) & 3 (CORR: phi k0-1 .. k0+2)
     issue(0, k0 - 1); issue(1, k0); issue(2, k0 + 1);
     issue_phi(k0 - 1); issue_phi(k0); issue_phi(k0 + 1); issue_phi(k0 + 2); issue_phi(k0 + 3);
+    issue_z(k0); issue_z(k0 + 1);
     cp_async_commit();
     cp_async_wait_all();
     if (CORR) __syncthreads();   // phi elements copied by other threads
@@ -779,6 +794,7 @@ __device__ __forceinline__ void k_tiled_body(const BC &bc, const StepArgs<T> &a,
         const bool more = k + 2 <= kend;
         const int snext = (k - k0 + 3) & 3;
         if (more) { issue(snext, k + 2); issue_phi(k + 4); }
+        issue_z(k + 2);
         cp_async_commit();
         const int sm_ = (k - k0) & 3, s0 = (k - k0 + 1) & 3, sp = (k - k0 + 2) & 3;
         if (active) {
@@ -793,7 +809,9 @@ __device__ __forceinline__ void k_tiled_body(const BC &bc, const StepArgs<T> &a,
             if (KIND == 1) {
                 nut_out[p] = nut_at<T>(a, q, i, j, k);
             } else {
-                stage_cell<T, LES, WM, KIND == 2>(a, q, Y, R, tau_x, tau_z, sc, i, j, k, uo, vo, wo, f1u, f1v, f1w, us, vs,
+                const T *zm = nullptr;
+                if constexpr (MS) zm = zmr[(k - k0) & 3];
+                stage_cell<T, LES, WM, KIND == 2>(a, q, Y, R, zm, tau_x, tau_z, sc, i, j, k, uo, vo, wo, f1u, f1v, f1w, us, vs,
                                                   wsf, rhs_only);
             }
         }
