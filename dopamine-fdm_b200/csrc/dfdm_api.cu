@@ -309,8 +309,6 @@ template <typename T> StepArgs<T> step_args(dfdm_ctx *c) {
     a.d = c->d;
     a.my = metric_view<T>(c->my_t, c->d.Ny);
     a.mz = metric_view<T>(c->mz_t, c->d.Nz);
-    a.myd = metric_view<double>(c->my_d, c->d.Ny);
-    a.mzd = metric_view<double>(c->mz_d, c->d.Nz);
     double inv_dx = 1.0 / c->dx;
     a.inv_dx = (T)inv_dx;
     a.dx2 = (T)(c->dx * c->dx);

@@ -71,14 +71,6 @@ __host__ __device__ __forceinline__ long long idx3(const Dims &d, int i, int j, 
 }
 __device__ __forceinline__ int wrap(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
 
-// U or W at a centre-in-y index j that may be a ghost (j = -1 or Ny); i, k already wrapped.
-template <typename T>
-__device__ __forceinline__ T ld_yc(const T *__restrict__ f, const Dims &d, int i, int j, int k) {
-    if (d.yper) { j = wrap(j, d.Ny); return __ldg(f + idx3(d, i, j, k)); }
-    if (j < 0) return -__ldg(f + idx3(d, i, 0, k));
-    if (j >= d.Ny) return -__ldg(f + idx3(d, i, d.Ny - 1, k));
-    return __ldg(f + idx3(d, i, j, k));
-}
 // V at a face-in-y index j in [-1, Ny-1] (walls) or any wrapped index (periodic)
 template <typename T>
 __device__ __forceinline__ T ld_yf(const T *__restrict__ f, const Dims &d, int i, int j, int k) {
@@ -86,14 +78,6 @@ __device__ __forceinline__ T ld_yf(const T *__restrict__ f, const Dims &d, int i
     if (j < 0) return T(0);
     return __ldg(f + idx3(d, i, j, k));
 }
-// nu_t at a centre-in-y index that may be a ghost: zero at the walls
-template <typename T>
-__device__ __forceinline__ T ld_nu(const T *__restrict__ f, const Dims &d, int i, int j, int k) {
-    if (d.yper) { j = wrap(j, d.Ny); return __ldg(f + idx3(d, i, j, k)); }
-    if (j < 0 || j >= d.Ny) return T(0);
-    return __ldg(f + idx3(d, i, j, k));
-}
-
 // x / d for a divisor whose correctly rounded reciprocal r = 1/d is at hand: Markstein's correction (P. W. Markstein,
 // "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).  The product
 // x r is within 1.5 ulp of the quotient; its remainder x - q d comes out of one fused multiply-add, and adding remainder

@@ -53,7 +53,6 @@ template <> struct RowProfile<double> {
 template <typename T> struct StepArgs {
     Dims d;
     Metric1D<T> my, mz;          // y and z metrics in the storage type
-    Metric1D<double> myd, mzd;   // the same in double (wall model, reductions)
     T inv_dx, dx2;
     int nwl;                     // divergence-form wall band (adv_wall_layers)
     int wm;                      // flat-wall EQWM on both no-slip walls
