@@ -591,17 +591,6 @@ template <typename T> struct Impl {
         CKL();
         return DFDM_OK;
     }
-    // the DCT-IV of every x line: 6 or 9 groups of 16 outputs per block, whichever pads the Nx outputs less
-    template <bool FWD> static int dct(dfdm_ctx *c, const T *in, T scale, T *out) {
-        const int N = c->d.Nx, lines = c->d.Ny * c->d.Nz, bl = 16 * dct_tl<T>();
-        auto blocks = [&](int nq) { return (N + 16 * nq - 1) / (16 * nq); };
-        const int nq = blocks(9) * 9 < blocks(6) * 6 ? 9 : 6;
-        const dim3 g((lines + bl - 1) / bl, blocks(nq));
-        if (nq == 9) k_dct<T, FWD, 9><<<g, 256, 0, c->stream>>>(N, lines, in, f(c->d_dct), scale, out);
-        else k_dct<T, FWD, 6><<<g, 256, 0, c->stream>>>(N, lines, in, f(c->d_dct), scale, out);
-        CKL();
-        return DFDM_OK;
-    }
     // dfdm_solve_poisson on a duct context: staging (rhs_p) -> phi -> x FFT -> z eigenmodes -> y solve per (kx, mode)
     // -> z^-1 -> x FFT^-1 -> staging.  The eigenmode transforms run out of place; the y solve works on whichever
     // buffer is the context's spectrum, so the two are swapped around it.
@@ -612,8 +601,10 @@ template <typename T> struct Impl {
         k_unpack_rhs_p<T><<<reduce_grid(d), 256, 0, st>>>(d, n1, n2, c->staging, f(c->phi));
         CKL();
         // x: the FFT, or with inflow/outflow x the DCT-IV (the duct of the reference's CPU build)
+        const int nbd = (d.Ny * d.Nz + DCT_LINES - 1) / DCT_LINES, ntd = (d.Nx + 31) / 32 * 32;
         if (c->xdct) {
-            if (int rc = dct<true>(c, f(c->phi), T(1), f(c->spec))) return rc;
+            k_dct_x<T><<<nbd, ntd, 0, st>>>(d, f(c->phi), f(c->d_dct), (C *)c->spec);
+            CKL();
         } else if (int rc = fwd_x(c, false, f(c->phi))) {
             return rc;
         }
@@ -633,7 +624,8 @@ template <typename T> struct Impl {
         }
         if (c->xdct) {
             const T inv_norm = (T)(1.0 / (2.0 * (double)d.Nx * (double)d.Nz));   // the nzp cancels the inverse matrix's
-            if (int rc = dct<false>(c, f(c->spec), inv_norm, f(c->phi))) return rc;
+            k_idct_x<T><<<nbd, ntd, 0, st>>>(d, (const C *)c->spec, f(c->d_dct), inv_norm, f(c->phi));
+            CKL();
         } else if (int rc = launch(c, 6, 1)) {
             return rc;
         }
@@ -649,11 +641,14 @@ template <typename T> struct Impl {
         const size_t n = (size_t)n1 * n2 * n3;
         k_unpack_rhs_p<T><<<reduce_grid(d), 256, 0, c->stream>>>(d, n1, n2, c->staging, f(c->phi));
         CKL();
-        if (int rc = dct<true>(c, f(c->phi), T(1), f(c->spec))) return rc;
+        const int nb = (d.Ny * d.Nz + DCT_LINES - 1) / DCT_LINES, nt = (d.Nx + 31) / 32 * 32;
+        k_dct_x<T><<<nb, nt, 0, c->stream>>>(d, f(c->phi), f(c->d_dct), (C *)c->spec);
+        CKL();
         for (int which : {3, 4, 5})
             if (int rc = launch(c, which, 1)) return rc;
         const T inv_norm = (T)(1.0 / (2.0 * (double)d.Nx * (double)d.Nz));
-        if (int rc = dct<false>(c, f(c->spec), inv_norm, f(c->phi))) return rc;
+        k_idct_x<T><<<nb, nt, 0, c->stream>>>(d, (const C *)c->spec, f(c->d_dct), inv_norm, f(c->phi));
+        CKL();
         k_pack_rhs_p_bc<T><<<(int)std::min<size_t>((n + 255) / 256, 148 * 8), 256, 0, c->stream>>>(d, n1, n2, n3, 0, 1,
                                                                                                    f(c->phi), c->staging);
         CKL();

@@ -325,111 +325,98 @@ __global__ void __launch_bounds__(YS_COLS) k_ysolve3(Dims d, typename cplx_t<T>:
 // CPU build plans and its GPU build forms through a zero-padded 4N-point FFT), as a product with the N x N matrix
 // C[k][n] of those coefficients (symmetric; built on the host in FP64 with the angle reduced exactly, stored in the
 // context's precision T).  N = nx - 1 is odd and can be prime (257), so the matrix product replaces a fast transform.
-// Forward: x lines (the real field, x fastest) to the spectrum's kx columns (imaginary parts zero, kx = 0..N-1); inverse: the
-// real parts of the spectrum's lines to the real field, times 1 / (2 N nzp) (the DCT-IV is its own inverse up to 2N).  Both
-// run as k_dct.
-constexpr int DCT_NMAX = 257;   // the longest line
-// A block of 256 threads forms 16 NQ outputs of 16 TL lines, a thread NQ outputs (16 apart) of TL lines in registers, from
-// DCT_KT values of every line and rows of C at a time in two shared-memory buffers, the next ones travelling in registers
-// meanwhile.  Sums run over n in order, in T.  Bound by the FMA pipe and by the last wave of blocks; the earlier form, a
-// thread per output on 16 lines, was bound by its loads (5 per 16 FMAs, here 8 per 48).  A whole solve at 257 x 128 x 128,
-// host transfers included, FP32 1639 -> 1596 us, FP64 1880 -> 1788.  At 45 % of the FMA pipe: 384 blocks on 296 places leave
-// the second wave a third full.  Half the lines per block (twice the blocks, 3 per SM) measured 1605 us, and the same kernel
-// for the z-eigenmode products lost to k_zeig in FP64 (1545 -> 1560 us).
-constexpr int DCT_KT = 8;
-template <typename T> __host__ __device__ constexpr int dct_tl() { return sizeof(T) == 4 ? 8 : 4; }
-template <typename T, bool FWD, int NQ>
-__global__ void __launch_bounds__(256, 2) k_dct(int N, int lines, const T *__restrict__ in, const T *__restrict__ M,
-                                                T scale, T *__restrict__ out) {
-    pdl_enter();
-    constexpr int TL = dct_tl<T>(), BL = 16 * TL, BQ = 16 * NQ, PA = BL + 4;
-    constexpr int NA = BL * DCT_KT / 256, NB = (BQ * DCT_KT + 255) / 256;   // elements per thread of a tile
-    struct alignas(16) Vec { T x[16 / sizeof(T)]; };
-    constexpr int W = 16 / (int)sizeof(T);
-    __shared__ __align__(16) T as[2][DCT_KT][PA];
-    __shared__ __align__(16) T bs[2][DCT_KT][BQ];
-    const int tq = threadIdx.x & 15, tv = threadIdx.x >> 4;
-    const int q0 = blockIdx.y * BQ;
-    const int v0 = blockIdx.x * BL;   // every index is below 2^31 (the cell count is below 2^31 / 3)
-    T ra[NA], rb[NB];
-    auto load = [&](int n0) {
+// A block stages DCT_LINES lines in shared memory as [n][line] (the lines' values at one n contiguous, read as
+// vectors at one address by every thread of a warp); thread t < N produces output t of all of them, reading row n of
+// C at consecutive t (coalesced, through L1) and accumulating in T.  Forward: x lines (the real field, x fastest) to
+// the spectrum's kx columns (imaginary parts zero, kx = 0..N-1); inverse: the real parts of the spectrum's lines to
+// the real field, times 1 / (2 N nzp) (the DCT-IV is its own inverse up to 2N).
+constexpr int DCT_LINES = 16, DCT_NMAX = 257, DCT_THREADS = 288;   // lines per block; the longest line; threads
+static_assert(DCT_THREADS >= (DCT_NMAX + 31) / 32 * 32, "one thread per output of the longest line");
+template <typename T> struct DctVec;
+template <> struct DctVec<float> { typedef float4 type; static constexpr int W = 4; };
+template <> struct DctVec<double> { typedef double2 type; static constexpr int W = 2; };
+template <typename T>
+__device__ __forceinline__ void dct_accumulate(T cv, const T *__restrict__ v, T (&acc)[DCT_LINES]) {
+    typedef typename DctVec<T>::type V;
+    constexpr int W = DctVec<T>::W;
 #pragma unroll
-        for (int e = 0; e < NA; ++e) {
-            const int a = threadIdx.x + e * 256;
-            const int n = a % DCT_KT, l = a / DCT_KT;
-            const int v = v0 + l, o = v * N + n0 + n;
-            ra[e] = n0 + n < N && v < lines ? in[FWD ? o : 2 * o] : T(0);
-        }
+    for (int q = 0; q < DCT_LINES / W; ++q) {
+        const V x = reinterpret_cast<const V *>(v)[q];
+        const T *xs = reinterpret_cast<const T *>(&x);
 #pragma unroll
-        for (int e = 0; e < NB; ++e) {
-            const int b = threadIdx.x + e * 256, n = b / BQ, q = b - n * BQ;
-            rb[e] = n < DCT_KT && n0 + n < N && q0 + q < N ? __ldg(M + (n0 + n) * N + q0 + q) : T(0);
-        }
-    };
-    auto store = [&](int buf) {
-#pragma unroll
-        for (int e = 0; e < NA; ++e) {
-            const int a = threadIdx.x + e * 256;
-            const int n = a % DCT_KT, l = a / DCT_KT;
-            as[buf][n][l] = ra[e];
-        }
-#pragma unroll
-        for (int e = 0; e < NB; ++e) {
-            const int b = threadIdx.x + e * 256, n = b / BQ;
-            if (n < DCT_KT) bs[buf][n][b - n * BQ] = rb[e];
-        }
-    };
-    T acc[TL][NQ];
-#pragma unroll
-    for (int l = 0; l < TL; ++l)
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) acc[l][q] = T(0);
-    load(0);
-    store(0);
-    __syncthreads();
-    for (int n0 = 0, buf = 0; n0 < N; n0 += DCT_KT, buf ^= 1) {
-        const bool more = n0 + DCT_KT < N;
-        if (more) load(n0 + DCT_KT);
-#pragma unroll
-        for (int n = 0; n < DCT_KT; ++n) {
-            T a[TL], b[NQ];
-#pragma unroll
-            for (int l = 0; l < TL; l += W) {
-                const Vec x = *reinterpret_cast<const Vec *>(&as[buf][n][tv * W + 16 * l]);
-#pragma unroll
-                for (int w = 0; w < W; ++w) a[l + w] = x.x[w];
-            }
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) b[q] = bs[buf][n][tq + 16 * q];
-#pragma unroll
-            for (int l = 0; l < TL; ++l)
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) acc[l][q] = fma(b[q], a[l], acc[l][q]);
-        }
-        if (more) {
-            store(buf ^ 1);   // last read before the previous barrier
-            __syncthreads();
-        }
-    }
-    const int o0 = q0 + tq;
-#pragma unroll
-    for (int l = 0; l < TL; ++l) {
-        const int v = v0 + tv * W + 16 * (l - l % W) + l % W;   // a thread's TL lines: TL / W groups of W, 16 W apart
-        if (v >= lines) continue;
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const int o = o0 + 16 * q;
-            if (o >= N) break;
-            if constexpr (FWD) {   // two stores: forming the pairs in registers spills
-                out[2 * (v * N + o)] = acc[l][q];
-                out[2 * (v * N + o) + 1] = T(0);
-            } else {
-                out[v * N + o] = acc[l][q] * scale;
-            }
-        }
+        for (int w = 0; w < W; ++w) acc[q * W + w] = fma(cv, xs[w], acc[q * W + w]);
     }
 }
-
+// acc[l] += sum_n col[n * N] * ln[n][l]: the column's coefficients are loaded DCT_AHEAD at a time, one group ahead of
+// the group being accumulated (the matrix is shared by every block and mostly served by L1).
+constexpr int DCT_AHEAD = 8;
+template <typename T>
+__device__ __forceinline__ void dct_column(const T *__restrict__ col, int N, const T *__restrict__ ln, T (&acc)[DCT_LINES]) {
+    T ca[DCT_AHEAD], cb[DCT_AHEAD];
+    auto load = [&](T (&c)[DCT_AHEAD], int n0) {
+#pragma unroll
+        for (int q = 0; q < DCT_AHEAD; ++q) c[q] = __ldg(col + (size_t)(n0 + q) * N);
+    };
+    auto proc = [&](const T (&c)[DCT_AHEAD], int n0) {
+#pragma unroll
+        for (int q = 0; q < DCT_AHEAD; ++q) dct_accumulate<T>(c[q], ln + (n0 + q) * DCT_LINES, acc);
+    };
+    const int full = N / DCT_AHEAD * DCT_AHEAD;
+    int n0 = 0;
+    if (full > 0) load(ca, 0);
+    for (; n0 + 2 * DCT_AHEAD <= full; n0 += 2 * DCT_AHEAD) {
+        load(cb, n0 + DCT_AHEAD);
+        proc(ca, n0);
+        if (n0 + 2 * DCT_AHEAD < full) load(ca, n0 + 2 * DCT_AHEAD);
+        proc(cb, n0 + DCT_AHEAD);
+    }
+    if (n0 < full) { proc(ca, n0); n0 += DCT_AHEAD; }
+    for (; n0 < N; ++n0) dct_accumulate<T>(__ldg(col + (size_t)n0 * N), ln + n0 * DCT_LINES, acc);
+}
+template <typename T>
+__global__ void __launch_bounds__(DCT_THREADS) k_dct_x(Dims d, const T *__restrict__ src, const T *__restrict__ C,
+                                                       typename cplx_t<T>::type *__restrict__ spec) {
+    pdl_enter();
+    __shared__ __align__(16) T ln[DCT_LINES * DCT_NMAX];
+    const int N = d.Nx, nlines = d.Ny * d.Nz;
+    const int line0 = blockIdx.x * DCT_LINES, nl = min(DCT_LINES, nlines - line0);
+    for (int e = threadIdx.x; e < DCT_LINES * N; e += blockDim.x) {
+        const int l = e / N, n = e - l * N;
+        ln[n * DCT_LINES + l] = l < nl ? src[(size_t)(line0 + l) * N + n] : T(0);
+    }
+    __syncthreads();
+    const int k = threadIdx.x;
+    if (k >= N) return;
+    T acc[DCT_LINES];
+#pragma unroll
+    for (int l = 0; l < DCT_LINES; ++l) acc[l] = T(0);
+    dct_column<T>(C + k, N, ln, acc);
+#pragma unroll
+    for (int l = 0; l < DCT_LINES; ++l)
+        if (l < nl) spec[(size_t)(line0 + l) * N + k] = mkc<T>(acc[l], T(0));
+}
+template <typename T>
+__global__ void __launch_bounds__(DCT_THREADS) k_idct_x(Dims d, const typename cplx_t<T>::type *__restrict__ spec,
+                                                        const T *__restrict__ C, T inv_norm, T *__restrict__ dst) {
+    pdl_enter();
+    __shared__ __align__(16) T ln[DCT_LINES * DCT_NMAX];
+    const int N = d.Nx, nlines = d.Ny * d.Nz;
+    const int line0 = blockIdx.x * DCT_LINES, nl = min(DCT_LINES, nlines - line0);
+    for (int e = threadIdx.x; e < DCT_LINES * N; e += blockDim.x) {
+        const int l = e / N, k = e - l * N;
+        ln[k * DCT_LINES + l] = l < nl ? spec[(size_t)(line0 + l) * N + k].x : T(0);
+    }
+    __syncthreads();
+    const int n = threadIdx.x;
+    if (n >= N) return;
+    T acc[DCT_LINES];
+#pragma unroll
+    for (int l = 0; l < DCT_LINES; ++l) acc[l] = T(0);
+    dct_column<T>(C + n, N, ln, acc);
+#pragma unroll
+    for (int l = 0; l < DCT_LINES; ++l)
+        if (l < nl) dst[(size_t)(line0 + l) * N + n] = acc[l] * inv_norm;
+}
 // The solved field back into rhs_p's shape for the Poisson-only contexts.  x: with periodic x (xwrap) the copies of
 // apply_periodic_xz_pressure (rhs_p(nxg-1) = rhs_p(2)) and of the next wrap for the plane nxg, as k_pack_rhs_p
 // writes them; with inflow/outflow x the plane nxg is left alone.  z: with periodic z (zwrap) the copy
