@@ -31,17 +31,17 @@ template <> __device__ __forceinline__ float bcast<float>(float2 x) { return x.x
 template <> __device__ __forceinline__ F2 bcast<F2>(float2 x) { return F2(x); }
 
 // Base-profile terms of one row (FP32; the profile is zero in FP64), from ub of rows j-1, j, j+1 (mirrored on wall ghost
-// rows).  f, fm: the profile at the y faces j and j-1; x: (1 + wd) ub; c: its diffusion's flux difference; dp, dm: its steps
-// across the two faces.
+// rows).  f: the profile at the y face j; df: its step from face j-1, f - fm with w0 + w1 = 1, formed from the steps dp and dm
+// across the two faces; x: (1 + wd) ub; c: its diffusion's flux difference.
 template <typename T> struct RowProfile {
-    T u, f, fm, x, c, dp, dm;
+    T u, f, df, x, c, dp, dm;
     template <typename Y> __device__ __forceinline__ void load(const T *ubr, const Y &y, T wd) {
         u = ubr[1];
         f = mad(y.w1(), ubr[2], mulv(y.w0(), ubr[1]));
-        fm = mad(y.w1m(), ubr[1], mulv(y.w0m(), ubr[0]));
         x = mad(wd, ubr[1], ubr[1]);
         dp = ubr[2] - ubr[1];
         dm = ubr[1] - ubr[0];
+        df = mad(y.w0m(), dm, mulv(y.w1(), dp));
         c = nmad(y.invfm(), dm, mulv(y.invf(), dp));
     }
 };
@@ -321,15 +321,16 @@ template <> __device__ __forceinline__ F2 wall_flux<F2>(const double *t) { retur
 // The reference writes each convective term as wd (a1 b1 - a0 b0) + wa b (a1 - a0), a the advected and b the advecting
 // velocity on the two faces, b = (b0 + b1)/2 and wa + wd = 1 (wa = 1/2 skew-symmetric, 0 divergence form and in the wall
 // band).  It is evaluated here in the equivalent forms with the fewest operations:
-//   a1 (wd b1 + m) - a0 (wd b0 + m), m = wa (b0 + b1)/2              where a1 - a0 needs no care,
-//   (wd b1 or a's total) (b1 - b0) + (a1 - a0)(p b0 + q b1)           where U is the one interpolated: FP32 then takes
-//     a1 - a0 from the stored deviations, without the cancellation of the mean flow,
+//   a1 (wd b1 + m) - a0 (wd b0 + m), m = wa (b0 + b1)/2              for vw and wv, which have no mean part,
+//   (wd b1 or a's total) (b1 - b0) + (a1 - a0)(p b0 + q b1)           where U takes part: FP32 then takes a1 - a0 from the
+//     stored deviations and the profile's own steps, without the cancellation of the mean flow.  On a smooth channel flow
+//     with 96 rows the u equation is 2.2e-7 from 64 bits that way; with the first form for uv it was 8.5e-7 (times as now),
 //   (a1 - a0) (wd (a1 + a0) + wa a)                                  for uu, vv, ww,
 // interpolations to the y face j and the z face k are shared by two equations each, with constant viscosity the two terms of
 // a flux are collected before its metric, and with an eddy viscosity each edge's shear flux is formed once.  About 160
 // operations per cell against 240 for the term by term form (which in FP64 had 24 divisions besides), and in FP64 with a
 // smaller error against 80-bit arithmetic (relative to a noisy channel's right-hand sides: u 1.8e-15 -> 1.4e-16, v and w
-// 1.7e-16 -> 1.6e-16), since fewer terms are rounded.  The stage kernels are bound by instruction issue at 16 warps per SM:
+// 1.7e-16 -> 1.6e-16; a smooth one's: u 7.2e-15 -> 2.4e-16), since fewer terms are rounded.  The stage kernels are bound by instruction issue at 16 warps per SM:
 // 256 x 192 x 256 cells went from 172 to 146 us (stage 1) and from 223 to 187 us (fused stage) in FP32, and the FP64 step
 // from 2.74 to 2.41 ms; the LES kernels on 96 x 64 x 96 cells take 20 us as before in FP32, 90 x 53 x 60 cells step in 195
 // against 224 us in FP64.
@@ -370,11 +371,10 @@ __device__ __forceinline__ void rhs_at(const SA &a, const Q &q, const AxisLocal<
         const T V0m = q.V(0, -1, 0), V1m = q.V(1, -1, 0), Ujm = q.Ud(0, -1, 0);
         const T W0m = q.W(0, 0, -1), W1m = q.W(1, 0, -1), Ukm = q.Ud(0, 0, -1);
         // y
-        const T vs1 = Vc + V10, vs0 = V0m + V1m, m = mulv(hq, vs0 + vs1);
-        T u1, u0;
-        if constexpr (PROF) { u1 = uy + R.f; u0 = mad(Y.w1m(), Uc, mad(Y.w0m(), Ujm, R.fm)); }
-        else { u1 = uy; u0 = mad(Y.w1m(), Uc, mulv(Y.w0m(), Ujm)); }
-        const T cy = nmad(u0, mad(hwd, vs0, m), mulv(u1, mad(hwd, vs1, m)));
+        const T vs1 = Vc + V10, vs0 = V0m + V1m;
+        T u1 = uy, duy = uy - mad(Y.w1m(), Uc, mulv(Y.w0m(), Ujm));
+        if constexpr (PROF) { u1 = u1 + R.f; duy = duy + R.df; }
+        const T cy = mad(duy, mad(hq, vs1, mulv(hp, vs0)), mulv(mulv(hwd, u1), vs1 - vs0));
         // z
         const T ws1 = Wc + W10, ws0 = W0m + W1m, uzm = mad(Z.w1m(), Uc, mulv(Z.w0m(), Ukm)), du = uz - uzm;
         T ut;

@@ -1,6 +1,7 @@
 """The right-hand sides of every form the stage kernels are compiled in (DNS, eddy viscosity, wall model; skew-symmetric and
 divergence form, with and without the wall band; periodic and wall-bounded y) on a grid with partial tiles in x and y, and
-the wall model on column counts around a block's, against the oracle: FP64 1e-12, FP32 1e-5 relative L2."""
+the wall model on column counts around a block's, against the oracle: FP64 1e-12, FP32 1e-5 relative L2.  Those fields are
+strongly perturbed; the FP32 arithmetic on a smooth mean flow has a test of its own, with a bound in units of its rounding."""
 import numpy as np
 import pytest
 
@@ -58,6 +59,46 @@ def test_right_hand_sides(oracle_mod, wall, sgs, wm, scheme, nwl):
         for key, n, a, b in zip("uvw", rows, s.compute_rhs(), want):
             assert rel_l2(a[:Nx, :n, :Nz], b[:Nx, :n, :Nz]) <= tol, (prec, variant, key)
         s.close()
+
+
+@pytest.mark.parametrize("scheme,wm", [(0, 0), (1, 0), (0, 1), (1, 1)])
+def test_mean_flow_does_not_cancel_in_fp32(oracle_mod, scheme, wm):
+    """The u right-hand side of U(y), V(y), W = 0, both exact in FP32, on rows much thinner than the profile changes over:
+    -d(uv)/dy is a small difference of large u v at the two faces.  Formed from the differences of u and of v its rounding is
+    relative to those: ten roundings at most lie between the stored values and each term (u or its step at the face from two
+    weights, three; its partner, two; their product, its metric and the metric's own rounding, three; the sums, two), so the
+    error is below 10 x 2^-24 times the sum of the terms' absolute values.  Formed from u v itself it is 4 to 5 times that bound."""
+    c = cases.Case(name="mean", nx=34, ny=193, nz=10, Lx_i=6.0, Ly_i=2.0, Lz_i=3.0, grid_type=2, alpha_grid=1.0, nu=1e-4,
+                   dt=1e-3, dPdx=1.0, sgs_model=0, flat_wall_model_flag=wm, advection_scheme=scheme,
+                   ic="poiseuille_uniform", ic_amplitude=18.0)
+    U, V, W, P = cases.initial_condition(c)
+    y = cases.faces(c)[1]
+    U[:] = U.astype(np.float32)
+    V[:] = np.sin(np.pi * y / 2.0).astype(np.float32)[None, :, None]
+    V[:, -1] = 0.0
+    cases.fill_ghosts(c, U, V, W)
+    o = oracle_mod.Oracle(c)
+    o.set_state(U, V, W, P)
+    if wm:
+        o.compute_wall_model(True)
+    Nx, Ny, Nz = c.cells
+    want = o.compute_rhs()[0][:Nx, 1:Ny - 1, :Nz]          # the wall rows hold the wall model's flux
+    g = np.concatenate([[-0.5 * y[1]], 0.5 * (y[1:] + y[:-1]), [2.0 * y[-1] - 0.5 * (y[-1] + y[-2])]])
+    u, v = U[1, :, 1], V[1, :, 1]                           # centres with ghosts, faces
+    w = (g[1:] - y) / (g[1:] - g[:-1])
+    uf, flux = w * u[:-1] + (1.0 - w) * u[1:], c.nu * np.abs(np.diff(u) / np.diff(g))
+    big = lambda a: np.maximum(np.abs(a[1:]), np.abs(a[:-1]))
+    terms = (np.abs(np.diff(uf)) * big(v) + big(uf) * np.abs(np.diff(v)) + flux[1:] + flux[:-1]) / np.diff(y) + abs(c.dPdx)
+    bound = 10.0 * 2.0 ** -24 * np.linalg.norm(np.broadcast_to(terms[None, 1:-1, None], want.shape))
+    for variant in (0, 1):
+        s = Solver(c, "fp32")
+        s.set_stage_variant(variant)
+        s.set_state(U, V, W, P)
+        if wm:
+            s.compute_wall_model(True)
+        got = s.compute_rhs()[0][:Nx, 1:Ny - 1, :Nz]
+        s.close()
+        assert np.linalg.norm(got - want) <= bound, (variant, np.linalg.norm(got - want) / bound)
 
 
 @pytest.mark.parametrize("columns", [60, 64, 72, 128])
