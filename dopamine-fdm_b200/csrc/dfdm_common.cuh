@@ -15,6 +15,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "div_by.h"
+
 namespace dfdm {
 
 // Programmatic dependent launch.  Every kernel of the library starts with pdl_enter(), which waits until the kernel
@@ -78,18 +80,6 @@ __device__ __forceinline__ T ld_yf(const T *__restrict__ f, const Dims &d, int i
     if (j < 0) return T(0);
     return __ldg(f + idx3(d, i, j, k));
 }
-// x / d for a divisor whose correctly rounded reciprocal r = 1/d is at hand: Markstein's correction (P. W. Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).  The product
-// x r is within 1.5 ulp of the quotient; its remainder x - q d comes out of one fused multiply-add, and adding remainder
-// times r leaves an error of half an ulp plus about 2^-52 ulp, so the result is the rounded quotient except where that
-// lies within 2^-52 ulp of a rounding boundary.  Finite operands whose quotient and remainder are normal numbers; an
-// infinite x gives NaN.  Three dependent operations in place of a divide, of which the FP64 stage kernels had about 24
-// per cell: 256 x 192 x 256 cells 3.45 -> 2.80 ms per FP64 step, 128 x 96 x 128 cells 0.51 -> 0.42 ms.
-__device__ __forceinline__ double div_by(double x, double d, double r) {
-    const double q = x * r;
-    return fma(fma(-q, d, x), r, q);
-}
-
 // Reciprocal helpers.  The tables hold 1/d rounded in double (FP64: what the reference's own 1/d gives) or rounded to
 // FP32 from it.
 template <typename T> struct Arith {
