@@ -56,6 +56,39 @@ def oracle_mod():
     return O
 
 
+def solve_bound(case):
+    """Relative L2 bound of an FP64 pressure solve with y walls: 1e-12, or for many rows the rounding of the pivots of its
+    lowest mode, 2^-53 of the largest diagonal entry of d2/dy2 (2/dy_min^2) over the smallest eigenvalue ((pi/Ly)^2)."""
+    from dfdm import cases
+    y = cases.faces(case)[1]
+    return max(1e-12, 2.0 ** -53 * 2.0 / np.diff(y).min() ** 2 / (np.pi / (y[-1] - y[0])) ** 2)
+
+
+def pressure_bounds(case, oracle_mod, state, want):
+    """Relative L2 bounds of P after some steps from `state`, `want` the oracle's state there, for a field whose first
+    projection removes much more than the later ones.  P is phi / (0.75 dt) of a weak phi, so what else phi sees counts.
+    FP64: the divergence that the first projection leaves, its solve's relative error, enters the next phi whole.
+    FP32: the same with eight roundings for the solve, and the rounding of u*: one rounding of the stored velocity (deviations
+    from the row means), projected, times sixteen for the operations of the stage update and of the divergence."""
+    from dfdm import cases
+    n = tuple(case.cells)
+    cut = lambda a: np.linalg.norm(a[:n[0], :n[1], :n[2]])
+
+    def phi(U, V, W):
+        o = oracle_mod.Oracle(case)
+        o.set_state(U, V, W, np.zeros_like(want[3]))
+        return cut(o.solve_poisson(o.divergence_rhs()))
+    phi2 = 0.75 * case.dt * np.linalg.norm(interior(case, "P", want[3]))
+    rng = np.random.default_rng(1)
+    noise = []
+    for key, a in zip("UVW", want):
+        dev = a - a.mean((0, 2), keepdims=True) if key == "U" else a
+        noise.append(np.asfortranarray(dev * rng.uniform(-1.0, 1.0, a.shape) * 2.0 ** -24))
+    cases.fill_ghosts(case, *noise)
+    phi1 = phi(*state[:3])
+    return {"fp64": solve_bound(case) * phi1 / phi2, "fp32": (8.0 * 2.0 ** -24 * phi1 + 16.0 * phi(*noise)) / phi2}
+
+
 def cfl_reference(c, U, V, W, nu_t, dt=None):
     """compute_cfl (src/monitor.f90:304-424) on the ghosted 1-based arrays: i = 2..nxg-1, j = 2..nyg-1,
     k = 2..nzg-1, written out in numpy (0-based slices)."""

@@ -1,10 +1,11 @@
 """The one-launch spectral solve of wall-bounded grids (k_plane: z transforms and tridiagonal solves of a kx plane in a pair
 of blocks) where its rule takes it and next to where it does not, against the oracle: the pressure solve and two steps, FP64
-1e-12, FP32 1e-5 relative L2; the launch count of a step tells which path ran (13 kernels with it, 19 without)."""
+1e-12, FP32 1e-5 relative L2, P after the steps at the bounds of pressure_bounds; the launch count of a step tells which path
+ran (13 kernels with it, 19 without)."""
 import numpy as np
 import pytest
 
-from conftest import rel_l2
+from conftest import interior, pressure_bounds, rel_l2
 from dfdm import cases
 from dfdm.native import Solver
 
@@ -39,6 +40,7 @@ def test_against_the_oracle(oracle_mod, shape, fp64, fp32):
     phi = o.solve_poisson(rhs)[:n[0], :n[1], :n[2]]
     o.step(2)
     want = o.get_state()
+    p_tol = pressure_bounds(c, oracle_mod, state, want)
     for prec, takes, tol in (("fp64", fp64, 1e-12), ("fp32", fp32, 1e-5)):
         s = Solver(c, prec)
         assert rel_l2(s.solve_poisson_equation(rhs)[:n[0], :n[1], :n[2]], phi) <= tol, prec
@@ -46,11 +48,11 @@ def test_against_the_oracle(oracle_mod, shape, fp64, fp32):
         before = s.launch_count()
         s.compute_time_step_RK3(2)
         assert s.launch_count() - before == 2 * (13 if takes else 19), prec
-        # P is left to the solve above: phi / (0.75 dt) of a weak pressure carries the rounding of the mean flow,
-        # 1e-16 u dx / dt = 4e-15 against P = 5e-3 here, times the smoothing of the solve (2e-12 to 7e-12 measured, with
-        # either path)
-        for key, a, b in zip("UVW", s.get_state(), want):
+        got = s.get_state()
+        for key, a, b in zip("UVW", got, want):
             assert rel_l2(a, b) <= tol, (prec, key)
+        err = rel_l2(interior(c, "P", got[3]), interior(c, "P", want[3]))
+        assert err <= p_tol[prec], (prec, "P", err, p_tol[prec])
         s.close()
 
 
