@@ -119,7 +119,6 @@ struct dfdm_ctx {
     double *zmd = nullptr, *ymd = nullptr;      // FP64: the same values per z plane and y row (StepArgs::zmd, ymd)
     void *zm8 = nullptr;                        // FP32: the z metrics of each plane in load_pairs order (StepArgs::zm8)
     double *d_wfac = nullptr;                   // LES + wall model: wall factors of the eddy viscosity (k_wall_sgs)
-    double *my_d = nullptr, *mz_d = nullptr;    // same in double
     void *tw_x = nullptr, *twr_x = nullptr, *tw_z = nullptr, *tw_y = nullptr;
     FFTPlan plan_x{}, plan_z{}, plan_y{};
     double *d_kxx = nullptr, *d_kzz = nullptr, *d_kyy = nullptr, *d_lo = nullptr, *d_di = nullptr, *d_up = nullptr;
@@ -273,7 +272,7 @@ template <typename T> Metric1D<T> metric_view(void *base, int N) {
     const int L = N + 3;
     T *b = (T *)base;
     Metric1D<T> m;
-    m.dc = b + 0 * L + 1; m.df = b + 1 * L + 1; m.w0 = b + 2 * L + 1; m.w1 = b + 3 * L + 1;
+    m.dc = b + 0 * L + 1; m.w0 = b + 2 * L + 1; m.w1 = b + 3 * L + 1;
     m.idc = b + 4 * L + 1; m.idf = b + 5 * L + 1;
     return m;
 }
@@ -1701,18 +1700,14 @@ int dfdm_create(const dfdm_grid *g, const dfdm_params *prm, dfdm_ctx **out) {
     build_metric(c->y, c->yg, c->ny, d.Ny, my);
     build_metric(c->z, c->zg, c->nz, d.Nz, mz);
     void *tmp = nullptr;
-    if ((rc = upload_as<double>(c, &tmp, my))) return bail(rc);
-    c->my_d = (double *)tmp;
-    if ((rc = upload_as<double>(c, &tmp, mz))) return bail(rc);
-    c->mz_d = (double *)tmp;
     // the eight metrics around index p of an axis with n cells: w0, w1 at p-1 and p, idc at p and p+1, idf at p-1 and p
     auto around = [](const std::vector<double> &m, int n, int p, int t) {
         const int src[8][2] = {{2, p - 1}, {3, p - 1}, {2, p}, {3, p}, {4, p}, {4, p + 1}, {5, p - 1}, {5, p}};
         return m[(size_t)src[t][0] * (n + 3) + 1 + src[t][1]];
     };
     if (c->prec == DFDM_FP64) {
-        c->my_t = c->my_d;
-        c->mz_t = c->mz_d;
+        if ((rc = upload_as<double>(c, &c->my_t, my))) return bail(rc);
+        if ((rc = upload_as<double>(c, &c->mz_t, mz))) return bail(rc);
         std::vector<double> zd((size_t)d.Nz * 8), yd((size_t)d.Ny * 8);
         for (int k = 0; k < d.Nz; ++k)
             for (int t = 0; t < 8; ++t) zd[(size_t)k * 8 + t] = around(mz, d.Nz, k, t);

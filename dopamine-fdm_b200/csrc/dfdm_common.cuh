@@ -54,9 +54,10 @@ template <typename T> __host__ __device__ __forceinline__ typename cplx_t<T>::ty
 //   dc[j] = y(j+2) - y(j+1)            width of centre j           ("y(j)-y(j-1)" in reference indices)
 //   df[j] = yg(j+3) - yg(j+2)          centre spacing across face j ("yg(j+1)-yg(j)")
 //   w0[j], w1[j] = weight_y_0(j+2), weight_y_1(j+2) of face j
-// plus reciprocals for the FP32 path.  z uses the same layout.  Stored in double and in the storage type.
+// and the reciprocals idc, idf of dc and df, rounded in double (what the reference's own 1/d gives) and in FP32 rounded from
+// that.  z uses the same layout.
 template <typename T> struct Metric1D {
-    const T *dc, *df, *w0, *w1, *idc, *idf;   // all offset by +1 (point at element 1 of the allocation)
+    const T *dc, *w0, *w1, *idc, *idf;   // all offset by +1 (point at element 1 of the allocation)
 };
 
 struct Dims {
@@ -80,12 +81,6 @@ __device__ __forceinline__ T ld_yf(const T *__restrict__ f, const Dims &d, int i
     if (j < 0) return T(0);
     return __ldg(f + idx3(d, i, j, k));
 }
-// Reciprocal helpers.  The tables hold 1/d rounded in double (FP64: what the reference's own 1/d gives) or rounded to
-// FP32 from it.
-template <typename T> struct Arith {
-    static __device__ __forceinline__ T inv(const T *, const T *id, int j) { return id[j]; }
-};
-
 // Asynchronous global -> shared copies (cp.async, 4 or 8 bytes per element).
 template <int B> __device__ __forceinline__ void cp_async(void *smem, const void *gmem) {
     unsigned s = (unsigned)__cvta_generic_to_shared(smem);

@@ -34,7 +34,6 @@ __device__ __forceinline__ void k_fwd_x2_body(const BC &bc, const PoissonArgs<T>
                                                 const typename cplx_t<T>::type *__restrict__ tw,
                                                 const typename cplx_t<T>::type *__restrict__ twr) {
     typedef typename cplx_t<T>::type C;
-    typedef Arith<T> A;
     constexpr int N1 = Split<M>::N1, N2 = Split<M>::N2, Nx = 2 * M;
     constexpr int LD = TR ? RowLayout<M>::LDT : RowLayout<M>::LD;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -60,7 +59,7 @@ __device__ __forceinline__ void k_fwd_x2_body(const BC &bc, const PoissonArgs<T>
         if constexpr (FROM_DIV) {
             const int k = (int)fdiv((unsigned)line, a.fNy), j = line - k * Ny;
             const bool vzero = (j == 0) && !d.yper;
-            const T riy = A::inv(a.my.dc, a.my.idc, j), riz = A::inv(a.mz.dc, a.mz.idc, k);
+            const T riy = a.my.idc[j], riz = a.mz.idc[k];
             const T *Ur = U + (size_t)line * Nx, *Vr = V + (size_t)line * Nx, *Wr = W_ + (size_t)line * Nx;
             const T *Vm = Vr + (vzero ? 0 : (j > 0 ? -Nx : (Ny - 1) * Nx)), *Wm = Wr + (k == 0 ? (Nz - 1) * plane : -plane);
 #pragma unroll 1

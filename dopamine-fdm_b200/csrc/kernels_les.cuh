@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(les::NT, 2) k_les(StepArgs<T> a, const T *__re
             off[q] = g * Nx + gi;
             if constexpr (CORR) {
                 pix[q] = jj * PXP + ii;
-                iyq[q] = (ghost[q] || g >= d.NyV) ? T(0) : Arith<T>::inv(a.my.df, a.my.idf, g);
+                iyq[q] = (ghost[q] || g >= d.NyV) ? T(0) : a.my.idf[g];
             }
         }
     }
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(les::NT, 2) k_les(StepArgs<T> a, const T *__re
         const int s = vslot(p);
         if constexpr (CORR) {   // project_velocity of the previous stage (k_correct's arithmetic)
             const T *p0 = smp + pslot(p) * PSP, *p1 = smp + pslot(p + 1) * PSP;
-            const T iz = Arith<T>::inv(a.mz.df, a.mz.idf, wrapz(p));
+            const T iz = a.mz.idf[wrapz(p)];
 #pragma unroll
             for (int q = 0; q < PER; ++q) {
                 if (off[q] < 0) continue;

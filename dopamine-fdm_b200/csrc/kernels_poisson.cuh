@@ -34,7 +34,6 @@ __global__ void __launch_bounds__(256) k_fwd_x(PoissonArgs<T> a, int lx, const T
                                                const typename cplx_t<T>::type *__restrict__ twr) {
     pdl_enter();
     typedef typename cplx_t<T>::type C;
-    typedef Arith<T> A;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const Dims &d = a.d;
     const int Nx = d.Nx, Ny = d.Ny, Nz = d.Nz, M = Nx / 2, plane = Nx * Ny;
@@ -55,7 +54,7 @@ __global__ void __launch_bounds__(256) k_fwd_x(PoissonArgs<T> a, int lx, const T
             T vjm;
             if (j > 0) vjm = __ldg(V + o - Nx);
             else vjm = d.yper ? __ldg(V + o + (Ny - 1) * Nx) : T(0);
-            T inv_dyj = A::inv(a.my.dc, a.my.idc, j), inv_dzk = A::inv(a.mz.dc, a.mz.idc, k);
+            T inv_dyj = a.my.idc[j], inv_dzk = a.mz.idc[k];
             val = (__ldg(U + o) - __ldg(U + oim)) * a.inv_dx + (__ldg(V + o) - vjm) * inv_dyj +
                   (__ldg(W + o) - __ldg(W + okm)) * inv_dzk;
         } else {
@@ -597,7 +596,6 @@ __global__ void __launch_bounds__(256) k_correct(PoissonArgs<T> a, const T *__re
                                                  T *__restrict__ V, T *__restrict__ W, T *__restrict__ P,
                                                  const T *__restrict__ uo, const T *__restrict__ vo, const T *__restrict__ wo) {
     pdl_enter();
-    typedef Arith<T> A;
     const Dims &d = a.d;
     const int Nx = d.Nx, Ny = d.Ny, Nz = d.Nz, plane = Nx * Ny;
     int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
@@ -609,12 +607,12 @@ __global__ void __launch_bounds__(256) k_correct(PoissonArgs<T> a, const T *__re
     T su = us[p], sw = ws[p];
     if (uo) { su = uo[p] + su; sw = wo[p] + sw; }
     U[p] = su - (pxp - pc) * a.inv_dx;
-    W[p] = sw - (pzp - pc) * A::inv(a.mz.df, a.mz.idf, k);
+    W[p] = sw - (pzp - pc) * a.mz.idf[k];
     if (j < d.NyV) {
         T pyp = __ldg(phi + (j == Ny - 1 ? p - (Ny - 1) * Nx : p + Nx));
         T sv = vs[p];
         if (uo) sv = vo[p] + sv;
-        V[p] = sv - (pyp - pc) * A::inv(a.my.df, a.my.idf, j);
+        V[p] = sv - (pyp - pc) * a.my.idf[j];
     }
     if (P) {
         const double pdiv = a.dtp ? *a.dtp * (3.0 / 4.0) : a.pdiv;
@@ -636,7 +634,6 @@ __device__ __forceinline__ void k_correct4_body(const BC &bc, const PoissonArgs<
                                                   T *__restrict__ V, T *__restrict__ W, T *__restrict__ P,
                                                   const T *__restrict__ uo, const T *__restrict__ vo, const T *__restrict__ wo) {
     typedef typename Vec4<T>::type V4;
-    typedef Arith<T> A;
     const Dims &d = a.d;
     const int Nx = d.Nx, Ny = d.Ny, Nz = d.Nz, plane = Nx * Ny, nq = Nx >> 2;
     const int iq = bc.idx().x * blockDim.x + threadIdx.x;
@@ -647,7 +644,7 @@ __device__ __forceinline__ void k_correct4_body(const BC &bc, const PoissonArgs<
     const V4 pc = *reinterpret_cast<const V4 *>(phi + p);
     const T pnext = __ldg(phi + (i + 4 == Nx ? p + 4 - Nx : p + 4));
     const V4 pz = *reinterpret_cast<const V4 *>(phi + (k == Nz - 1 ? p - (Nz - 1) * plane : p + plane));
-    const T idx = a.inv_dx, idz = A::inv(a.mz.df, a.mz.idf, k);
+    const T idx = a.inv_dx, idz = a.mz.idf[k];
     V4 u = *reinterpret_cast<const V4 *>(us + p), w = *reinterpret_cast<const V4 *>(ws + p);
     if (uo) {   // increment form: u* = uo + du, rounded as the stage kernel rounds it
         const V4 bu = *reinterpret_cast<const V4 *>(uo + p), bw = *reinterpret_cast<const V4 *>(wo + p);
@@ -662,7 +659,7 @@ __device__ __forceinline__ void k_correct4_body(const BC &bc, const PoissonArgs<
     *reinterpret_cast<V4 *>(W + p) = w;
     if (j < d.NyV) {
         const V4 py = *reinterpret_cast<const V4 *>(phi + (j == Ny - 1 ? p - (Ny - 1) * Nx : p + Nx));
-        const T idy = A::inv(a.my.df, a.my.idf, j);
+        const T idy = a.my.idf[j];
         V4 v = *reinterpret_cast<const V4 *>(vs + p);
         if (vo) {
             const V4 bv = *reinterpret_cast<const V4 *>(vo + p);

@@ -125,12 +125,11 @@ __device__ __forceinline__ double wall_gradient_factor(double u_c, double w_c, b
 template <typename T, typename Q>
 __device__ __forceinline__ T nut_at(const StepArgs<T> &a, const Q &q, int i, int j, int k) {
     const Dims &d = a.d;
-    typedef Arith<T> A;
     const Metric1D<T> &my = a.my, &mz = a.mz;
     T dz_c = mz.dc[k], dz2 = dz_c * dz_c;
-    T inv_dz_k = A::inv(mz.dc, mz.idc, k), inv_zg_km = A::inv(mz.df, mz.idf, k - 1), inv_zg_kp = A::inv(mz.df, mz.idf, k);
+    T inv_dz_k = mz.idc[k], inv_zg_km = mz.idf[k - 1], inv_zg_kp = mz.idf[k];
     T dy_c = my.dc[j], dy2_c = dy_c * dy_c;
-    T inv_yg_jm = A::inv(my.df, my.idf, j - 1), inv_yg_jp = A::inv(my.df, my.idf, j), inv_dy_j = A::inv(my.dc, my.idc, j);
+    T inv_yg_jm = my.idf[j - 1], inv_yg_jp = my.idf[j], inv_dy_j = my.idc[j];
     T inv_dx = a.inv_dx, dx2 = a.dx2;
     T Uc = q.U(0, 0, 0), Um = q.U(-1, 0, 0);
     T a11 = (Uc - Um) * inv_dx;
@@ -300,8 +299,8 @@ __global__ void __launch_bounds__(WALL_THREADS) k_wall_sgs(StepArgs<T> a, const 
         const T pkm = phi[idx3(d, i, j, km)], pkp = phi[idx3(d, i, j, kp)];
         u0 = u0 - (pc - pm) * a.inv_dx;
         u1 = u1 - (pp - pc) * a.inv_dx;
-        w0 = w0 - (pc - pkm) * Arith<T>::inv(a.mz.df, a.mz.idf, km);
-        w1 = w1 - (pkp - pc) * Arith<T>::inv(a.mz.df, a.mz.idf, k);
+        w0 = w0 - (pc - pkm) * a.mz.idf[km];
+        w1 = w1 - (pkp - pc) * a.mz.idf[k];
     }
     const T ubj = a.ub[j];
     const T Um = u0 + ubj, Uc = u1 + ubj;   // as TileQ::U forms them
@@ -688,7 +687,7 @@ __device__ __forceinline__ void k_tiled_body(const BC &bc, const StepArgs<T> &a,
             off[q] = g * Nx + gi;
             if constexpr (CORR) {
                 pix[q] = jj * PXP + ii;
-                iyq[q] = (ghost[q] || g >= d.NyV) ? T(0) : Arith<T>::inv(a.my.df, a.my.idf, g);
+                iyq[q] = (ghost[q] || g >= d.NyV) ? T(0) : a.my.idf[g];
             }
         }
     }
@@ -737,7 +736,7 @@ __device__ __forceinline__ void k_tiled_body(const BC &bc, const StepArgs<T> &a,
         if constexpr (CORR) {   // project_velocity of the previous stage (k_correct's arithmetic)
             const int kw = k < 0 ? k + Nz : (k >= Nz ? k - Nz : k);
             const int p0 = (k - k0 + 1) % 5, p1 = (k - k0 + 2) % 5;
-            const T iz = Arith<T>::inv(a.mz.df, a.mz.idf, kw);
+            const T iz = a.mz.idf[kw];
 #pragma unroll
             for (int q = 0; q < PER; ++q) {
                 if (off[q] < 0) continue;
@@ -942,7 +941,7 @@ __device__ __forceinline__ void k_tiled2_body(const BC &bc, const StepArgs<float
             off[q] = g * Nx + gi;
             if constexpr (CORR) {
                 pix[q] = jj * PXP + ii;
-                iyq[q] = (ghost[q] || g >= d.NyV) ? 0.0f : Arith<float>::inv(a.my.df, a.my.idf, g);
+                iyq[q] = (ghost[q] || g >= d.NyV) ? 0.0f : a.my.idf[g];
             }
         }
     }
@@ -994,7 +993,7 @@ __device__ __forceinline__ void k_tiled2_body(const BC &bc, const StepArgs<float
         if constexpr (CORR) {   // project_velocity of the previous stage (k_correct's arithmetic, lane by lane)
             const int kw = k < 0 ? k + Nz : (k >= Nz ? k - Nz : k);
             const int p0 = (k - k0 + 1) % 5, p1 = (k - k0 + 2) % 5;
-            const float iz = Arith<float>::inv(a.mz.df, a.mz.idf, kw);
+            const float iz = a.mz.idf[kw];
 #pragma unroll
             for (int q = 0; q < PER; ++q) {
                 if (off[q] < 0) continue;

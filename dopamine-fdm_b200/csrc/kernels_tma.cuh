@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(256, 2) k_tma2(StepArgs<float> a, const __grid
         const int s = slot_of(p);
         const int pw = p < 0 ? p + Nz : (p >= Nz ? p - Nz : p);
         const int s1 = slot_of(p + 1);   // CORR: phi(p+1) for the w correction
-        const float iz = CORR ? Arith<float>::inv(a.mz.df, a.mz.idf, pw) : 0.0f;
+        const float iz = CORR ? a.mz.idf[pw] : 0.0f;
         for (int e = threadIdx.x; e < NPAIR * BY; e += 256) {
             const int r = e / NPAIR, c = 2 + 2 * (e - r * NPAIR);
             const int yg = j0 - 1 + r;
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(256, 2) k_tma2(StepArgs<float> a, const __grid
                 u.x = u.x - (pc.y - pc.x) * a.inv_dx; u.y = u.y - (pn - pc.y) * a.inv_dx;
                 w.x = w.x - (pz.x - pc.x) * iz; w.y = w.y - (pz.y - pc.y) * iz;
                 if (yg < d.NyV) {
-                    const float iy = Arith<float>::inv(a.my.df, a.my.idf, yg);
+                    const float iy = a.my.idf[yg];
                     const float2 py = raw2(P0, P0l, P0r, c, r + 1);
                     v.x = v.x - (py.x - pc.x) * iy; v.y = v.y - (py.y - pc.y) * iy;
                 }
