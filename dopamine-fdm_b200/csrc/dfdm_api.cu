@@ -413,6 +413,7 @@ template <typename T, int M> constexpr size_t row_smem(int lx) {
 }
 // ---- k_plane: where it runs and how ----
 const size_t PLANE_SMEM_MAX = 232448;   // shared memory a block may use on sm_100
+const int B200_SMS = 148;               // for plane_wins, which dfdm_footprint_bytes asks without a device
 // threads of a block: equal rounds of the first pass's items, at least the sweeps' 2 Nz
 int plane_block(const Dims &d) {
     int n2 = 1;
@@ -434,11 +435,41 @@ bool plane_wins(const Dims &d, int prec) {
     const size_t sm = prec == DFDM_FP64 ? plane_smem<double>(d.Ny, d.Nz) : plane_smem<float>(d.Ny, d.Nz);
     if (sm > PLANE_SMEM_MAX) return false;
     if (d.Nxc > 49 && d.Ny * d.Nz < 48 * 48) return false;
-    return d.Nz < 256 || (d.Nxc >= 33 && 2 * d.Nxc <= 148);
+    return d.Nz < 256 || (d.Nxc >= 33 && 2 * d.Nxc <= B200_SMS);
 }
 // blocks of a column transform of `nl` columns each: the (j, kx) columns of the z transforms (families 3, 5) or the
 // (kz, kx) columns of the periodic-y solve (family 4)
 int col_blocks(const Dims &d, int which, int nl) { return (d.Nxc * (which == 4 ? d.Nz : d.Ny) + nl - 1) / nl; }
+
+// Programmatic dependent launch in the captured steps: every kernel-to-kernel edge of the graph becomes a
+// programmatic edge (the destination may be scheduled once every block of the source has started, and waits in
+// pdl_enter for the source's completion).  An edge the runtime does not accept as programmatic stays as it was.
+int make_programmatic(cudaGraph_t g) {
+    size_t n = 0;
+    if (cudaGraphGetEdges_v2(g, nullptr, nullptr, nullptr, &n) != cudaSuccess) { cudaGetLastError(); return DFDM_OK; }
+    std::vector<cudaGraphNode_t> from(n), to(n);
+    std::vector<cudaGraphEdgeData> ed(n);
+    if (n == 0 || cudaGraphGetEdges_v2(g, from.data(), to.data(), ed.data(), &n) != cudaSuccess) {
+        cudaGetLastError();
+        return DFDM_OK;
+    }
+    for (size_t i = 0; i < n; ++i) {
+        cudaGraphNodeType a, b;
+        if (cudaGraphNodeGetType(from[i], &a) != cudaSuccess || cudaGraphNodeGetType(to[i], &b) != cudaSuccess) continue;
+        if (a != cudaGraphNodeTypeKernel || b != cudaGraphNodeTypeKernel || ed[i].type != cudaGraphDependencyTypeDefault)
+            continue;
+        cudaGraphEdgeData pe;
+        std::memset(&pe, 0, sizeof(pe));
+        pe.type = cudaGraphDependencyTypeProgrammatic;
+        pe.from_port = cudaGraphKernelNodePortProgrammatic;
+        CK(cudaGraphRemoveDependencies_v2(g, &from[i], &to[i], &ed[i], 1));
+        if (cudaGraphAddDependencies_v2(g, &from[i], &to[i], &pe, 1) != cudaSuccess) {
+            cudaGetLastError();
+            CK(cudaGraphAddDependencies_v2(g, &from[i], &to[i], &ed[i], 1));
+        }
+    }
+    return DFDM_OK;
+}
 
 template <typename T> struct Impl {
     typedef typename cplx_t<T>::type C;
@@ -898,9 +929,13 @@ template <typename T> struct Impl {
         return DFDM_OK;
     }
 
-    // Autotuner of the FP32 stage kernel: times the variants on this grid (a stage-2 launch, 2 warm-up + 5 timed;
-    // the TMA variant where the grid allows it) and keeps the fastest.  The choice is cached per device, grid shape and model flags for the process, so a
-    // serving loop that opens many contexts of one shape pays the timing once.
+    // Autotuner of the FP32 stage kernel: times the variants on this grid (the TMA variant where the grid allows it) and
+    // keeps the fastest.  A window is two steps' stage launches (stage 1 and, with fused corrections, the fused stages 2 and
+    // 3) replayed as a graph, as a step launches them; the variants' windows alternate, and the least time of each counts.
+    // Single windows of five stage-2 launches on the stream measured the launch rate on small grids: at 32^3 both variants
+    // read 6.5 to 6.8 us, so either was chosen, where a step takes 57.4 us with the one and 61.4 with the other and a group
+    // of 16 cases 113 to 124 against 125 to 135.  The choice is cached per device, grid shape and model flags for the
+    // process, so a serving loop that opens many contexts of one shape pays the timing once.
     static int tune_stage(dfdm_ctx *c, bool force) {
         if constexpr (sizeof(T) == 8) { (void)force; c->stage_variant = 0; return DFDM_OK; }
         int dev = 0;
@@ -915,32 +950,59 @@ template <typename T> struct Impl {
             for (int v = 0; v < 3; ++v) c->stage_ms[v] = it->second.ms[v];
             return DFDM_OK;
         }
-        StageCoef sc{2, 0.0, c->prm.dt, 0.25, 5.0 / 12.0, 0};
-        // the variants are those of the stage kernel that reads a stored eddy viscosity (k_les has one form)
-        struct Restore { dfdm_ctx *c; bool v; ~Restore() { c->sgs_tile = v; } } restore{c, c->sgs_tile};
+        const StageCoef sc{2, 0.0, c->prm.dt, 0.25, 5.0 / 12.0, 0};
+        // the variants are those of the stage kernel that reads a stored eddy viscosity (k_les has one form); the launches go
+        // to the context's own stream (a caller's may not be one that can be captured)
+        struct Restore {
+            dfdm_ctx *c; bool tile; cudaStream_t st; cudaEvent_t e[2] = {}; cudaGraph_t g[3] = {}; cudaGraphExec_t x[3] = {};
+            ~Restore() {
+                c->sgs_tile = tile;
+                c->stream = st;
+                for (auto q : x) if (q) cudaGraphExecDestroy(q);
+                for (auto q : g) if (q) cudaGraphDestroy(q);
+                for (auto q : e) if (q) cudaEventDestroy(q);
+            }
+        } r{c, c->sgs_tile, c->stream};
         c->sgs_tile = false;
-        cudaEvent_t e0, e1;
-        CK(cudaEventCreate(&e0));
-        CK(cudaEventCreate(&e1));
-        int rc = DFDM_OK;
-        for (int v = 0; v < (c->tma_ok ? 3 : 2) && !rc; ++v) {
+        c->stream = c->own_stream;
+        for (auto &e : r.e) CK(cudaEventCreate(&e));
+        const int nv = c->tma_ok ? 3 : 2, launches = 6;
+        double best[3] = {-1.0, -1.0, -1.0};
+        auto window = [&](int v, double *ms) {
+            CK(cudaEventRecord(r.e[0], c->stream));
+            CK(cudaGraphLaunch(r.x[v], c->stream));
+            CK(cudaEventRecord(r.e[1], c->stream));
+            CK(cudaEventSynchronize(r.e[1]));
+            float t = 0.0f;
+            CK(cudaEventElapsedTime(&t, r.e[0], r.e[1]));
+            *ms = t;
+            return DFDM_OK;
+        };
+        double ms = 0.0;
+        for (int v = 0; v < nv; ++v) {
             c->stage_variant = v;
-            for (int r = 0; r < 2 && !rc; ++r) rc = stage_kernel(c, sc, nullptr);
-            if (rc) break;
-            cudaEventRecord(e0, c->stream);
-            for (int r = 0; r < 5 && !rc; ++r) rc = stage_kernel(c, sc, nullptr);
-            cudaEventRecord(e1, c->stream);
-            if (cudaEventSynchronize(e1) != cudaSuccess) rc = fail(DFDM_ERR_CUDA, "stage-kernel tuning failed");
-            float ms = 0.0f;
-            cudaEventElapsedTime(&ms, e0, e1);
-            c->stage_ms[v] = ms / 5.0;
+            CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+            int rc = DFDM_OK;
+            for (int q = 0; q < launches && !rc; ++q)
+                rc = c->fused && !c->les ? launch(c, 1, q % 3 + 1) : stage_kernel(c, sc, nullptr);
+            const cudaError_t e = cudaStreamEndCapture(c->stream, &r.g[v]);
+            if (rc) return rc;
+            CK(e);
+            if ((rc = make_programmatic(r.g[v]))) return rc;
+            CK(cudaGraphInstantiate(&r.x[v], r.g[v], 0));
+            if ((rc = window(v, &ms))) return rc;   // warm-up
         }
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        if (rc) return rc;
+        const int windows = std::max(1, std::min(6, (int)(0.4 / ms) + 1));   // the larger the grid, the fewer
+        for (int q = 0; q < windows; ++q)
+            for (int v = 0; v < nv; ++v) {
+                if (int rc = window(v, &ms)) return rc;
+                if (best[v] < 0.0 || ms < best[v]) best[v] = ms;
+            }
         c->stage_variant = 0;
-        for (int v = 1; v < 3; ++v)
-            if (c->stage_ms[v] > 0.0 && c->stage_ms[v] < c->stage_ms[c->stage_variant]) c->stage_variant = v;
+        for (int v = 0; v < nv; ++v) {
+            c->stage_ms[v] = best[v] / launches;
+            if (c->stage_ms[v] < c->stage_ms[c->stage_variant]) c->stage_variant = v;
+        }
         g_tune[key] = TuneEntry{c->stage_variant, {c->stage_ms[0], c->stage_ms[1], c->stage_ms[2]}};
         return DFDM_OK;
     }
@@ -2201,36 +2263,6 @@ int dfdm_set_landing_times(dfdm_ctx *c, int n, const double *t_land) {
 }
 
 // ---- the step ----
-// Programmatic dependent launch in the captured steps: every kernel-to-kernel edge of the graph becomes a
-// programmatic edge (the destination may be scheduled once every block of the source has started, and waits in
-// pdl_enter for the source's completion).  An edge the runtime does not accept as programmatic stays as it was.
-static int make_programmatic(cudaGraph_t g) {
-    size_t n = 0;
-    if (cudaGraphGetEdges_v2(g, nullptr, nullptr, nullptr, &n) != cudaSuccess) { cudaGetLastError(); return DFDM_OK; }
-    std::vector<cudaGraphNode_t> from(n), to(n);
-    std::vector<cudaGraphEdgeData> ed(n);
-    if (n == 0 || cudaGraphGetEdges_v2(g, from.data(), to.data(), ed.data(), &n) != cudaSuccess) {
-        cudaGetLastError();
-        return DFDM_OK;
-    }
-    for (size_t i = 0; i < n; ++i) {
-        cudaGraphNodeType a, b;
-        if (cudaGraphNodeGetType(from[i], &a) != cudaSuccess || cudaGraphNodeGetType(to[i], &b) != cudaSuccess) continue;
-        if (a != cudaGraphNodeTypeKernel || b != cudaGraphNodeTypeKernel || ed[i].type != cudaGraphDependencyTypeDefault)
-            continue;
-        cudaGraphEdgeData pe;
-        std::memset(&pe, 0, sizeof(pe));
-        pe.type = cudaGraphDependencyTypeProgrammatic;
-        pe.from_port = cudaGraphKernelNodePortProgrammatic;
-        CK(cudaGraphRemoveDependencies_v2(g, &from[i], &to[i], &ed[i], 1));
-        if (cudaGraphAddDependencies_v2(g, &from[i], &to[i], &pe, 1) != cudaSuccess) {
-            cudaGetLastError();
-            CK(cudaGraphAddDependencies_v2(g, &from[i], &to[i], &ed[i], 1));
-        }
-    }
-    return DFDM_OK;
-}
-
 static int step_n(dfdm_ctx *c, int nsteps) {
     for (int n = 0; n < nsteps; ++n) {
         double to = c->t;

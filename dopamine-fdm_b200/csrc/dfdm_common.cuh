@@ -9,7 +9,7 @@
 // y is periodic (Ny cells, wrap) or bounded by no-slip walls (Ny cells): then the ghost centre j = -1 / Ny of U
 // and W holds minus the first / last interior value (apply_Robin_bc_y with alpha = 0), V's wall faces j = -1 and
 // j = Ny-1 are zero (row Ny-1 is stored and never written), and nu_t's ghosts are zero (sgs_fill_ghosts).
-// The spectral array is complex, (Nx/2+1) x Ny x Nz, kx fastest.
+// The spectral array is complex, (Nx/2+1) x Ny x Nz, kx fastest; where k_plane runs, y fastest and kx slowest.
 #pragma once
 
 #include <cuda_runtime.h>

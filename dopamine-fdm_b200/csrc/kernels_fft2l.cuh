@@ -2,9 +2,10 @@
 //
 // Same operations, inputs and outputs as the Stockham kernels of kernels_poisson.cuh (k_fwd_x, k_col_fft, k_inv_x):
 // only the transform itself is organised differently.  Step 1 of the z transforms reads its operands straight from
-// global memory and their step 2 writes straight to global memory, so a column crosses shared memory once.  The x
-// transforms fill shared memory first, with coalesced loads (the forward one with the divergence pairs, the inverse one
-// with the packed half-length spectrum), and form the modes k and M-k together.
+// global memory and their step 2 writes straight to global memory, so a column crosses shared memory once.  The forward x
+// transform fills shared memory first, with coalesced loads of the divergence, and forms the modes k and M-k together; the
+// inverse one forms the packed half-length spectrum in registers straight from global memory (staged through shared memory
+// the same way it took 32 us at 256 x 192 x 256 cells in FP32, and 29 us like this).
 #pragma once
 
 #include "fft_reg.cuh"

@@ -8,7 +8,9 @@
 // function the per-case kernel runs, given a JobBlock instead of the hardware block registers) with the job's
 // arguments.  A job's arithmetic therefore depends on its own case only, never on the other jobs of the launch.  It is
 // the per-case kernel's source; the two compilations may contract scalar multiply-adds differently, so a case agrees
-// with its per-case steps to rounding.  The transform families are templated on their length, so a group launches
+// with its per-case steps to rounding.  One family differs: a wall-bounded context whose own steps run k_plane (the
+// elimination from both walls, kernels_plane.cuh) takes the three launches with the elimination from the lower wall in a
+// group, from a pivot table of its own.  The transform families are templated on their length, so a group launches
 // them once per distinct length.
 #pragma once
 

@@ -323,16 +323,16 @@ template <> __device__ __forceinline__ F2 wall_flux<F2>(const double *t) { retur
 //   a1 (wd b1 + m) - a0 (wd b0 + m), m = wa (b0 + b1)/2              for vw and wv, which have no mean part,
 //   (wd b1 or a's total) (b1 - b0) + (a1 - a0)(p b0 + q b1)           where U takes part: FP32 then takes a1 - a0 from the
 //     stored deviations and the profile's own steps, without the cancellation of the mean flow.  On a smooth channel flow
-//     with 96 rows the u equation is 2.2e-7 from 64 bits that way; with the first form for uv it was 8.5e-7 (times as now),
+//     with 96 rows the u equation is 2.2e-7 from 64 bits that way; with the first form for uv it was 8.5e-7, no faster,
 //   (a1 - a0) (wd (a1 + a0) + wa a)                                  for uu, vv, ww,
 // interpolations to the y face j and the z face k are shared by two equations each, with constant viscosity the two terms of
 // a flux are collected before its metric, and with an eddy viscosity each edge's shear flux is formed once.  About 160
 // operations per cell against 240 for the term by term form (which in FP64 had 24 divisions besides), and in FP64 with a
 // smaller error against 80-bit arithmetic (relative to a noisy channel's right-hand sides: u 1.8e-15 -> 1.4e-16, v and w
-// 1.7e-16 -> 1.6e-16; a smooth one's: u 7.2e-15 -> 2.4e-16), since fewer terms are rounded.  The stage kernels are bound by instruction issue at 16 warps per SM:
-// 256 x 192 x 256 cells went from 172 to 146 us (stage 1) and from 223 to 187 us (fused stage) in FP32, and the FP64 step
-// from 2.74 to 2.41 ms; the LES kernels on 96 x 64 x 96 cells take 20 us as before in FP32, 90 x 53 x 60 cells step in 195
-// against 224 us in FP64.
+// 1.7e-16 -> 1.6e-16; a smooth one's: u 7.2e-15 -> 2.4e-16), since fewer terms are rounded.  The stage kernels are bound by
+// instruction issue at 16 warps per SM: 256 x 192 x 256 cells went from 172 to 146 us (stage 1) and from 223 to 187 us (fused
+// stage) in FP32, and the FP64 step from 2.74 to 2.41 ms; the LES kernels on 96 x 64 x 96 cells take 20 us as before in FP32,
+// 90 x 53 x 60 cells step in 195 against 224 us in FP64.
 template <typename T, bool LES, bool WM, typename Q, typename SA, typename ZM>
 __device__ __forceinline__ void rhs_at(const SA &a, const Q &q, const AxisLocal<T> &Y, const RowProfile<T> &R, const ZM &Z,
                                        const double *__restrict__ tau_x, const double *__restrict__ tau_z, int i, int j,

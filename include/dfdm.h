@@ -187,7 +187,8 @@ int dfdm_solve_poisson_noalloc(dfdm_ctx *ctx, const double *rhs_p_in, double *ph
  * 1 computes two x-neighbour cells per thread with the packed FP32x2 instructions on 64 x 8 tiles, 2 is variant 1
  * with its z-plane tiles brought in by the Tensor Memory Accelerator (3-D boxes completing on mbarriers, four planes
  * in flight); variant 2 needs walls in y and Nx a multiple of 4. dfdm_create times the eligible variants on the
- * context's grid and keeps the fastest; the choice is cached per device and grid shape for the process.
+ * context's grid (a step's stage launches, replayed as a graph) and keeps the fastest; the choice is cached per device
+ * and grid shape for the process.
  * set_stage_variant forces 0, 1 or 2 (DFDM_ERR_UNSUPPORTED where not eligible), or re-times with -1 (FP64
  * contexts have variant 0 only); a change drops the context's captured step graph. get_stage_variant returns the
  * variant in use and the timings of variants 0 and 1, get_stage_timing that of any variant (ms per launch, -1
