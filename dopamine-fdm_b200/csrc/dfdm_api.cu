@@ -930,12 +930,13 @@ template <typename T> struct Impl {
     }
 
     // Autotuner of the FP32 stage kernel: times the variants on this grid (the TMA variant where the grid allows it) and
-    // keeps the fastest.  A window is two steps' stage launches (stage 1 and, with fused corrections, the fused stages 2 and
-    // 3) replayed as a graph, as a step launches them; the variants' windows alternate, and the least time of each counts.
-    // Single windows of five stage-2 launches on the stream measured the launch rate on small grids: at 32^3 both variants
-    // read 6.5 to 6.8 us, so either was chosen, where a step takes 57.4 us with the one and 61.4 with the other and a group
-    // of 16 cases 113 to 124 against 125 to 135.  The choice is cached per device, grid shape and model flags for the
-    // process, so a serving loop that opens many contexts of one shape pays the timing once.
+    // keeps the fastest.  A window is the stage launches of one step (four steps up to 2^20 cells), stage 1 and, with fused
+    // corrections, the fused stages 2 and 3, replayed as a graph as a step launches them; the variants' windows alternate,
+    // and the least time of each counts.  Single windows of five stage-2 launches on the stream measured the launch rate on
+    // small grids: at 32^3 both variants read 6.5 to 6.8 us (4.9 and 5.3 now), so either was chosen, where a step takes
+    // 57.4 us with the one and 61.4 with the other and a group of 16 cases 113 to 124 against 125 to 135.  The choice is
+    // cached per device, grid shape and model flags for the process, so a serving loop that opens many contexts of one shape
+    // pays the timing once.
     static int tune_stage(dfdm_ctx *c, bool force) {
         if constexpr (sizeof(T) == 8) { (void)force; c->stage_variant = 0; return DFDM_OK; }
         int dev = 0;
@@ -966,7 +967,7 @@ template <typename T> struct Impl {
         c->sgs_tile = false;
         c->stream = c->own_stream;
         for (auto &e : r.e) CK(cudaEventCreate(&e));
-        const int nv = c->tma_ok ? 3 : 2, launches = 6;
+        const int nv = c->tma_ok ? 3 : 2, launches = c->d.cells <= (1 << 20) ? 12 : 3;
         double best[3] = {-1.0, -1.0, -1.0};
         auto window = [&](int v, double *ms) {
             CK(cudaEventRecord(r.e[0], c->stream));
@@ -992,7 +993,7 @@ template <typename T> struct Impl {
             CK(cudaGraphInstantiate(&r.x[v], r.g[v], 0));
             if ((rc = window(v, &ms))) return rc;   // warm-up
         }
-        const int windows = std::max(1, std::min(6, (int)(0.4 / ms) + 1));   // the larger the grid, the fewer
+        const int windows = std::max(1, std::min(8, (int)(0.2 / ms) + 1));   // the larger the grid, the fewer
         for (int q = 0; q < windows; ++q)
             for (int v = 0; v < nv; ++v) {
                 if (int rc = window(v, &ms)) return rc;
