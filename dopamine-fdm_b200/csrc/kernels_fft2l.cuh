@@ -26,8 +26,8 @@ template <int Q> struct RowGroup {
 // Phase A forms the packed half-length line z_n = x_2n + i x_2n+1 in shared memory from 16-byte loads (every two-level
 // length makes Nx a multiple of 16, so rows and vectors are aligned); the two register steps follow in place.  It is bound
 // by the latency of its phases more than by bandwidth: pairs of cells with per-pair indexing and two buffers (fewer lines
-// per block) took 62 us at 256 x 192 x 256 cells in FP32 and 145 us in FP64, this form 46 and 105 us (207 MB of traffic in
-// FP32: 0.69 of the measured copy bandwidth).
+// per block) took 62 us at 256 x 192 x 256 cells in FP32 and 145 us in FP64, this form 46 to 49 and 110 us (202 MB in FP32:
+// 0.62 to 0.67 of the measured copy bandwidth).
 template <typename T, bool FROM_DIV, int M, bool TR = false, class BC>
 __device__ __forceinline__ void k_fwd_x2_body(const BC &bc, const PoissonArgs<T> &a, int lx, const T *__restrict__ U, const T *__restrict__ V,
                                                 const T *__restrict__ W_, const T *__restrict__ src,

@@ -5,10 +5,10 @@
 // plane.  Where half a plane and its pivots fit in a block's shared memory this kernel does all three in one launch: a
 // cluster of two blocks reads the plane once, each block its half of the y rows, keeps it in shared memory through the
 // passes and writes it once, in place of three launches that each read and write the whole spectrum (k_col2 / k_ysolve3 /
-// k_col2).  It is bound by the latency of its passes (6.3 MB in and out per launch at 128 x 96 x 128 cells in FP32, 45 % issue
-// on the SMs it uses), so it pays where the three launches are latency-bound too (plane_wins in dfdm_api.cu has the rule and
-// the timings).  One block per plane sweeping top to bottom took 21.6 us there against 32 for the three launches; the pair
-// of blocks brought the step from 197 to 182 us more.
+// k_col2).  It is bound by the latency of its passes (at 128 x 96 x 128 cells in FP32 6.4 MB of spectrum in and out and 6.4 MB
+// of pivots in 16.6 us, the blocks issuing in 31 % of their SMs' active cycles), so it pays where the three launches are
+// latency-bound too (plane_wins in dfdm_api.cu has the rule and the timings).  One block per plane sweeping top to bottom took
+// 21.6 us there against 32 for the three launches; the pair of blocks brought the step from 197 to 182 us more.
 //
 // Layout.  The spectrum of a context that runs this kernel is plane-major, spec[kx][line] with line = k*Ny + j, so a plane is
 // contiguous; the x transforms read and write it that way (their TR form).  In shared memory row `slot` holds one kz (or

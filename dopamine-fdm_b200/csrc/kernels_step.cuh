@@ -187,8 +187,8 @@ struct WallState {
 // (:442-583), smooth Reichardt law, matching height = first centre.  One thread per wall face of one set: blockIdx.z is
 // 2 iw + set, wall iw 0 lower or 1 upper, set 0 the U faces or 1 the W faces, so that every face's Newton solve (a serial
 // chain of FP64 logarithms, exponentials and divisions) runs in a thread of its own.  With one thread per (i, k) taking all
-// four solves in turn, behind a separate filter kernel, the two launches took 22 us at 96 x 96 columns; this one takes
-// 7 us.
+// four solves in turn, behind a separate filter kernel, the two launches took 23 us at 96 x 96 columns; this one takes
+// 8 us.
 constexpr int WALL_THREADS = 64;
 template <typename T>
 __global__ void __launch_bounds__(WALL_THREADS) k_wall_model(StepArgs<T> a, WallState ws, const T *__restrict__ U,
